@@ -208,6 +208,11 @@ struct gfk_plan {
     std::vector<int> chunk_begin;  // row chunks [chunk_begin[c], chunk_begin[c+1])
     std::vector<int> chunk_max_nk;
     int64_t rem_capacity = 0;  // complex values
+    // per-frequency grids: items of kc wavenumbers (RowItems), their rows and
+    // each row's first item, over the whole plan
+    int kc = 0;
+    std::vector<int> item_row, row_begin;
+    int *d_item_row = nullptr, *d_row_begin = nullptr;
     // device
     gfk::LayerP* d_lp = nullptr;
     gfk::MediumP* d_media = nullptr;
@@ -262,7 +267,7 @@ void plan_free(gfk_plan* p) {
     if (p->ev_chunk) cudaEventDestroy(p->ev_chunk);
     void* ptrs[] = {p->d_lp, p->d_media,  p->d_fd, p->d_ranges, p->d_lc,     p->d_wc2,    p->d_C,
                     p->d_rem, p->d_G,     p->d_status, p->d_A, p->d_rowexp, p->d_rowmax, p->d_partial,
-                    p->d_ksum, p->d_queue};
+                    p->d_ksum, p->d_queue, p->d_item_row, p->d_row_begin};
     for (void* q : ptrs)
         if (q) cudaFreeAsync(q, s);
     p->wts.reset();  // the weights go with their last plan (or stay in the context's cache)
@@ -516,6 +521,10 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         }
         p->tc = p->shared;
     }
+    // a single row has no weights to share (its sum costs less than a table of
+    // them plus a GEMM), and a single range takes the per-frequency sum
+    if (mode == kGridSingle || (p->nf == 1 && !p->tc && (nr > gfk::fused_max_ranges() || s->formulation != GFK_DUNKIN)))
+        p->shared = p->tc = false;
     // a few ranges on a shared grid: fuse the sum into the Dunkin propagator
     if (p->shared && s->formulation == GFK_DUNKIN && nr <= gfk::fused_max_ranges() && mode == kGridMulti) {
         p->fused = true;
@@ -547,6 +556,32 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
     p->chunk_max_nk.push_back(cmax);
     p->rem_capacity = cap;
 
+    int max_items = 0;
+    if (!p->shared) {
+        long long total = 0;
+        for (const auto& d : p->fd) total += d.kfar > 0 ? d.nk : 0;
+        p->kc = gfk::rows_item_size(total, nr);
+        // a chunk's partial sums (items x ranges) stay within 256 MB, or at one item a row
+        long long most = 0, rows = 0;
+        for (size_t c = 0; c + 1 < p->chunk_begin.size(); c++) {
+            long long t = 0;
+            for (int f = p->chunk_begin[c]; f < p->chunk_begin[c + 1]; f++) t += p->fd[f].nk;
+            most = std::max(most, t);
+            rows = std::max<long long>(rows, p->chunk_begin[c + 1] - p->chunk_begin[c]);
+        }
+        while (p->kc < (1 << 20) && p->kc < p->max_nk && (most / p->kc + rows) * nr * (int64_t)sizeof(cd) > (256ll << 20))
+            p->kc *= 2;
+        p->row_begin.reserve(p->nf + 1);
+        for (int f = 0; f < p->nf; f++) {
+            p->row_begin.push_back((int)p->item_row.size());
+            const int n = p->fd[f].kfar > 0 ? p->fd[f].nk : 0;
+            p->item_row.insert(p->item_row.end(), (n + p->kc - 1) / p->kc, f);
+        }
+        p->row_begin.push_back((int)p->item_row.size());
+        for (size_t c = 0; c + 1 < p->chunk_begin.size(); c++)
+            max_items = std::max(max_items, p->row_begin[p->chunk_begin[c + 1]] - p->row_begin[p->chunk_begin[c]]);
+    }
+
     // device buffers
     int st = GFK_OK;
     const size_t nfa = std::max(p->nf, 1);
@@ -568,6 +603,11 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         if (!st) st = dalloc(ctx, &p->d_partial, (size_t)max_cnf * nkb * nr);
     } else if (!st) {
         st = dalloc(ctx, &p->d_rem, (size_t)std::max<int64_t>(cap, 1));
+    }
+    if (!p->shared) {
+        if (!st) st = dalloc(ctx, &p->d_item_row, p->item_row.size());
+        if (!st) st = dalloc(ctx, &p->d_row_begin, p->row_begin.size());
+        if (!st) st = dalloc(ctx, &p->d_ksum, (size_t)max_items * nr);
     }
     if (!st && p->shared && !p->tc) {
         if (!(st = plan_weights(p, false, g_n, g_kmax / g_n, sizeof(double) * (size_t)g_n * nr)))
@@ -604,6 +644,8 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
     if (!st) st = h2d(ctx, p->d_media, p->media.data(), p->media.size());
     if (!st) st = h2d(ctx, p->d_fd, p->fd.data(), p->fd.size());
     if (!st) st = h2d(ctx, p->d_ranges, p->ranges.data(), nr);
+    if (!st && !p->shared) st = h2d(ctx, p->d_item_row, p->item_row.data(), p->item_row.size());
+    if (!st && !p->shared) st = h2d(ctx, p->d_row_begin, p->row_begin.data(), p->row_begin.size());
     if (!st && cudaStreamSynchronize(ctx->stream) != cudaSuccess)  // host tables may be freed by the caller
         st = fail(ctx, GFK_ECUDA, "plan upload failed");
     if (st) {
@@ -614,9 +656,9 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
     int nchunks = 0;
     for (size_t c = 0; c + 1 < p->chunk_begin.size(); c++)
         if (p->chunk_begin[c + 1] > p->chunk_begin[c]) nchunks++;
-    p->launches_per_exec = p->nf > 0 ? 2 + 2 * nchunks : 0;
-    if (p->nf > 0 && p->ksplit > 1) p->launches_per_exec += nchunks;
-    if (p->fused) p->prop_variant = 0;  // one launch shape; nothing to tune
+    p->launches_per_exec = p->nf > 0 ? (p->shared ? 2 : 1) + 2 * nchunks : 0;
+    if (p->nf > 0 && (p->ksplit > 1 || !p->shared)) p->launches_per_exec += nchunks;
+    if (p->fused || !p->shared) p->prop_variant = 0;  // one launch shape; nothing to tune
     *out = p;
     return GFK_OK;
 }
@@ -625,6 +667,12 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
 // maxima in d_rowmax[0, 2 rows), its finished-block counts after them.
 gfk::SliceOut slice_out(const gfk_plan* p, int rows) {
     return gfk::SliceOut{p->d_rowmax, p->d_rowmax + 2 * (size_t)rows, p->d_rowexp, p->d_A, p->Mp, p->Kp};
+}
+
+// The items of rows [fb, fb + n).
+gfk::RowItems row_items(const gfk_plan* p, int fb, int n) {
+    const int i0 = p->row_begin[fb];
+    return gfk::RowItems{p->d_item_row + i0, p->d_row_begin + fb, fb, i0, p->row_begin[fb + n] - i0, p->kc};
 }
 
 // Times every Dunkin launch shape on a window of up to 1024 rows of the first
@@ -767,7 +815,7 @@ int plan_enqueue(gfk_plan* p, bool timed) {
     if (timed && (st = begin_seg(p, 2, &seg))) return st;
     gfk::launch_layer_consts_fl(s, p->d_lp, p->d_media, p->d_fd, nf, p->max_nl, p->solve.omega_imag, form, p->d_lc,
                                 p->d_wc2);
-    gfk::launch_static(s, p->d_lc, p->d_media, p->d_fd, p->d_wc2, nf, form, p->d_C, p->d_status);
+    if (p->shared) gfk::launch_static(s, p->d_lc, p->d_media, p->d_fd, p->d_wc2, nf, form, p->d_C, p->d_status);
     // the Hankel weights depend only on the plan's grid and ranges: built by
     // the first execute of the first plan that holds them, kept for later
     // executes and plans (and out of a captured graph)
@@ -781,7 +829,7 @@ int plan_enqueue(gfk_plan* p, bool timed) {
         p->wts->built = true;
     }
     if (timed && (st = end_seg(p, seg))) return st;
-    ctx->launches += 2;
+    ctx->launches += p->shared ? 2 : 1;
     if (timed && p->prop_variant < 0 && (st = tune_prop(p))) return st;
     const double dk = p->shared ? p->g_kmax / p->g_n : 0.0;
     for (size_t c = 0; c + 1 < p->chunk_begin.size(); c++) {
@@ -796,6 +844,20 @@ int plan_enqueue(gfk_plan* p, bool timed) {
                                    p->d_G + (size_t)fb * p->nr);
             if (timed && (st = end_seg(p, seg))) return st;
             ctx->launches += 2;
+            if ((st = copy_chunk_out(p, fb, cnf))) return st;
+            continue;
+        }
+        if (!p->shared) {
+            const gfk::RowItems it = row_items(p, fb, cnf);
+            if (timed && (st = begin_seg(p, 0, &seg))) return st;
+            gfk::launch_prop_rows(s, p->d_lc, p->d_media, p->d_fd + fb, cnf, p->d_wc2 + fb, p->d_C + fb, form, p->d_rem,
+                                  p->d_status + fb, it);
+            if (timed && (st = end_seg(p, seg))) return st;
+            if (timed && (st = begin_seg(p, 1, &seg))) return st;
+            gfk::launch_quad_rows(s, p->d_rem, p->d_C + fb, p->d_ranges, cnf, p->nr, p->d_fd + fb, it, p->d_ksum,
+                                  p->d_G + (size_t)fb * p->nr);
+            if (timed && (st = end_seg(p, seg))) return st;
+            ctx->launches += 3;
             if ((st = copy_chunk_out(p, fb, cnf))) return st;
             continue;
         }
@@ -816,13 +878,10 @@ int plan_enqueue(gfk_plan* p, bool timed) {
                                     p->ksplit, p->d_ksum, std::max(p->tc_variant, 0)))
                 return fail(ctx, GFK_ECUDA, "tensor-core quadrature launch setup failed");
             ctx->launches += 1 + (p->ksplit > 1 ? 1 : 0);
-        } else if (p->shared) {
+        } else {
             gfk::launch_quad_gemm(s, p->d_rem, p->d_W, p->d_C + fb, p->d_ranges, cnf, p->g_n, p->nr, dk,
                                   p->d_G + (size_t)fb * p->nr, p->ksplit, p->d_ksum);
             ctx->launches += p->ksplit > 1 ? 1 : 0;
-        } else {
-            gfk::launch_quad_ragged(s, p->d_rem, p->d_C + fb, p->d_ranges, cnf, p->nr, p->d_fd + fb,
-                                    p->d_G + (size_t)fb * p->nr);
         }
         if (timed && (st = end_seg(p, seg))) return st;
         ctx->launches += p->tc ? 1 : 2;
@@ -1261,9 +1320,6 @@ int gfk_vertical_displacement(gfk_ctx* ctx, const gfk_medium* m, const gfk_solve
     gfk_plan* p = nullptr;
     int st = plan_one(ctx, m, s, &range_m, 1, &freq_hz, 1, opt, kGridSingle, &p);
     if (st) return st;
-    // a single range always takes the per-frequency (sequential-sum) quadrature
-    p->shared = false;
-    p->tc = false;
     st = plan_exec(p);
     int32_t fst = 0;
     if (!st) st = plan_download(p, out, &fst);

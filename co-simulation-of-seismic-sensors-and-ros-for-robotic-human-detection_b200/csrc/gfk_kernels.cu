@@ -7,10 +7,12 @@
 //                   static-subtracted integrand k u - C (fk.go:534-544)
 //   k_j0_table      the shared-grid Hankel weights w_i J0(k_i r_j) dk (fk.go:540-546)
 //   k_quad_gemm     the shared-grid wavenumber sum as an FP64 complex x real GEMM
-//   k_quad_ragged   per-frequency grids: the same sum with J0 in the loop
+//   k_quad_rows     per-frequency grids: the same sum with J0 in the loop, over
+//                   items of a row's wavenumbers
 //   k_bank_pack     FP64 [f][r] -> float32 range-major bank payload
 //                   (internal/bank/format.go:185-193)
 #include "gfk_kernels.cuh"
+#include "gfk_j0.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -95,11 +97,9 @@ __device__ __forceinline__ bool finite_cd(cd a) { return isfinite(a.re) && isfin
 
 // ------------------------------------------------------ static coefficient --
 
-__global__ void k_static(const LayerC* __restrict__ lc, const MediumP* __restrict__ media,
-                         const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2, int nf, int formulation,
-                         cd* __restrict__ C, int* __restrict__ status) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nf) return;
+__device__ __forceinline__ void static_row(const LayerC* __restrict__ lc, const MediumP* __restrict__ media,
+                                           const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2, int f,
+                                           int formulation, cd* __restrict__ C, int* __restrict__ status) {
     const FreqDesc d = fd[f];
     const double k = d.kfar;
     if (!(k > 0)) {
@@ -121,6 +121,13 @@ __global__ void k_static(const LayerC* __restrict__ lc, const MediumP* __restric
         c = mk(0.0);
     }
     C[f] = c;
+}
+
+__global__ void k_static(const LayerC* __restrict__ lc, const MediumP* __restrict__ media,
+                         const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2, int nf, int formulation,
+                         cd* __restrict__ C, int* __restrict__ status) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f < nf) static_row(lc, media, fd, wc2, f, formulation, C, status);
 }
 
 void launch_static(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, const cd* wc2, int nf,
@@ -166,7 +173,7 @@ __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const M
     }
     const int n = fdesc.kfar > 0 ? fdesc.nk : 0;
     const double d = fdesc.dk;
-    const cd c = C[f];
+    const cd c = C ? C[f] : mk(0.0);
     const cd w2 = wc2[f];
     cd* row = rem + fdesc.off;
     int bad = 0;
@@ -260,6 +267,33 @@ __global__ __launch_bounds__(THREADS, MINB) void k_prop(const LayerC* __restrict
     __shared__ PropSmem<THREADS, SLICE> sm;
     prop_item<FORM, THREADS, ILP, SWEEPS, SLICE>(lc, media, fd, wc2, C, rem, status, so, blockIdx.y, blockIdx.x,
                                                  gridDim.x, true, sm);
+}
+
+// Rows of uneven length: block (item, y) serves the y-th run of 128
+// wavenumbers of that item. A grid over (longest row, rows) is mostly empty
+// blocks when the rows differ a hundredfold (2.46M blocks for 57k runs on the
+// loam bank). The static coefficients are solved beside the integrand, by the
+// blocks past the last item: one solve is a serial chain (89 us alone in the
+// direct formulation), so the integrand is stored as k u and the sum takes
+// C off.
+template <int FORM>
+__global__ __launch_bounds__(128, FORM == 0 ? 1 : 5) void k_prop_rows(const LayerC* __restrict__ lc,
+                                                                     const MediumP* __restrict__ media,
+                                                                     const FreqDesc* __restrict__ fd, int nf,
+                                                                     const cd* __restrict__ wc2, cd* __restrict__ C,
+                                                                     cd* __restrict__ ku, int* __restrict__ status,
+                                                                     RowItems it) {
+    __shared__ PropSmem<128, false> sm;
+    const int item = blockIdx.x;
+    if (item >= it.items) {
+        const int f = (item - it.items) * 128 + threadIdx.x;
+        if (blockIdx.y == 0 && f < nf) static_row(lc, media, fd, wc2, f, FORM, C, status);
+        return;
+    }
+    const int f = it.row ? it.row[item] - it.row0 : 0;
+    const int run = (item - (it.begin ? it.begin[f] - it.item0 : 0)) * (it.kc / 128) + blockIdx.y;
+    if (run * 128 >= fd[f].nk) return;
+    prop_item<FORM, 128, 1, 1, false>(lc, media, fd, wc2, nullptr, ku, status, SliceOut{}, f, run, 0, true, sm);
 }
 
 // Persistent: items (f, run) in row order from q.next (zero at launch), so a
@@ -378,6 +412,16 @@ void launch_prop(cudaStream_t s, const LayerC* lc, const MediumP* media, const F
     } else {
         fn<<<dim3(runs, nf), v.threads, 0, s>>>(lc, media, fd, wc2, C, rem, status, so, PropQueue{});
     }
+}
+
+void launch_prop_rows(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, int nf,
+                      const cd* wc2, cd* C, int formulation, cd* ku, int* status, const RowItems& it) {
+    if (nf <= 0) return;
+    const dim3 grid(it.items + (nf + 127) / 128, it.kc / 128);
+    if (formulation == 0)
+        k_prop_rows<0><<<grid, 128, 0, s>>>(lc, media, fd, nf, wc2, C, ku, status, it);
+    else
+        k_prop_rows<1><<<grid, 128, 0, s>>>(lc, media, fd, nf, wc2, C, ku, status, it);
 }
 
 // ------------------------------------------------- fused propagator + sum --
@@ -726,38 +770,111 @@ void launch_quad_finish(cudaStream_t s, const cd* part, int splits, const cd* C,
 }
 
 // ---------------------------------------------- per-frequency-grid sum --
-// The reference's own order: the boundary term, then i = 1..n in sequence
-// (fk.go:529-548), one range per thread.
+//
+// Rows whose grids differ share no weight table: J0 is evaluated in the loop
+// (fk.go:529-548), so the FP64 pipe bounds the sum (about 35 instructions per
+// wavenumber and range for J0, 2 for the sum). One block serves one item (kc
+// consecutive wavenumbers of one row) and RT ranges: its threads run over the
+// wavenumbers, so the lanes of a warp take the same J0 branch, and each loads
+// an integrand value once for RT ranges; then a fixed-order reduction and one
+// partial per (item, range), which k_rows_finish adds in item order
+// (deterministic). Items, not rows, are the unit because row lengths differ a
+// hundredfold (a low bin's step is set by its own k/8Q): one thread per range
+// walking its row took 242 ms on a 614-bin x 270-range loam bank (7.3M
+// wavenumbers), most of it one block per SM on the longest rows.
 
-__global__ __launch_bounds__(128) void k_quad_ragged(const cd* __restrict__ rem, const cd* __restrict__ C,
-                                                     const double* __restrict__ ranges, int nf, int nr,
-                                                     const FreqDesc* __restrict__ fd, cd* __restrict__ G) {
-    const int f = blockIdx.y;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nr) return;
+constexpr int kRowThreads = 128;
+
+template <int RT>
+__global__ __launch_bounds__(kRowThreads) void k_quad_rows(const cd* __restrict__ ku, const cd* __restrict__ C,
+                                                          const double* __restrict__ ranges, int nr,
+                                                          const FreqDesc* __restrict__ fd, RowItems it,
+                                                          cd* __restrict__ part) {
+    __shared__ double s_red[kRowThreads / 32][2 * RT];
+    const int tiles = (nr + RT - 1) / RT;
+    const int item = blockIdx.x / tiles, tid = threadIdx.x;
+    const int f = it.row ? it.row[item] - it.row0 : 0;
+    const int first = (item - (it.begin ? it.begin[f] - it.item0 : 0)) * it.kc;
     const FreqDesc fdesc = fd[f];
-    const int n = fdesc.kfar > 0 ? fdesc.nk : 0;
+    const int n = fdesc.nk, last = min(first + it.kc, n);
     const double d = fdesc.dk;
-    const double r = ranges[j];
-    const cd c = C[f];
-    cd acc = c / r - (0.5 * d) * c;
-    const cd* row = rem + fdesc.off;
-    for (int i = 1; i <= n; i++) {
-        const double k = (double)i * d;
-        const double w = i == n ? 0.5 : 1.0;
-        const double wt = (w * j0(k * r)) * d;
-        const cd v = row[i - 1];
-        acc.re = fma(wt, v.re, acc.re);
-        acc.im = fma(wt, v.im, acc.im);
+    const int r0 = (blockIdx.x - item * tiles) * RT, nv = min(RT, nr - r0);
+    double r[RT], acc[2 * RT];
+#pragma unroll
+    for (int q = 0; q < RT; q++) {
+        r[q] = q < nv ? ranges[r0 + q] : 0.0;
+        acc[2 * q] = acc[2 * q + 1] = 0.0;
     }
-    G[(size_t)f * nr + j] = acc;
+    const cd* row = ku + fdesc.off;
+    const cd c = C[f];
+    for (int i = first + tid + 1; i <= last; i += kRowThreads) {
+        const double k = (double)i * d;
+        const cd v = (row[i - 1] - c) * (i == n ? 0.5 * d : d);
+#pragma unroll
+        for (int q = 0; q < RT; q++)
+            if (q < nv) {
+                const double w = j0_(k * r[q]);
+                acc[2 * q] = fma(w, v.re, acc[2 * q]);
+                acc[2 * q + 1] = fma(w, v.im, acc[2 * q + 1]);
+            }
+    }
+#pragma unroll
+    for (int q = 0; q < 2 * RT; q++)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
+    if ((tid & 31) == 0)
+#pragma unroll
+        for (int q = 0; q < 2 * RT; q++) s_red[tid >> 5][q] = acc[q];
+    __syncthreads();
+    if (tid < 2 * nv) {
+        double t = s_red[0][tid];
+#pragma unroll
+        for (int w = 1; w < kRowThreads / 32; w++) t += s_red[w][tid];
+        reinterpret_cast<double*>(part)[2 * ((size_t)item * nr + r0) + tid] = t;
+    }
 }
 
-void launch_quad_ragged(cudaStream_t s, const cd* rem, const cd* C, const double* ranges, int nf, int nr,
-                        const FreqDesc* fd, cd* G) {
-    if (nf <= 0) return;
-    dim3 grid((nr + 127) / 128, nf);
-    k_quad_ragged<<<grid, 128, 0, s>>>(rem, C, ranges, nf, nr, fd, G);
+__global__ void k_rows_finish(const cd* __restrict__ part, const cd* __restrict__ C,
+                              const double* __restrict__ ranges, int nf, int nr, const FreqDesc* __restrict__ fd,
+                              RowItems it, cd* __restrict__ G) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)nf * nr) return;
+    const int f = (int)(t / nr), j = (int)(t - (long long)f * nr);
+    const int b = it.begin ? it.begin[f] - it.item0 : 0;
+    const int e = it.begin ? it.begin[f + 1] - it.item0 : it.items;
+    cd acc = mk(0.0);
+#pragma unroll 8
+    for (int i = b; i < e; i++) acc += part[(size_t)i * nr + j];
+    const cd c = C[f];
+    G[t] = (c / ranges[j] - (0.5 * fd[f].dk) * c) + acc;  // fk.go:529-532
+}
+
+void launch_quad_rows(cudaStream_t s, const cd* ku, const cd* C, const double* ranges, int nf, int nr,
+                      const FreqDesc* fd, const RowItems& it, cd* part, cd* G) {
+    if (nf <= 0 || nr <= 0) return;
+    if (it.items > 0) {
+        // 8 ranges per block: one integrand load and one reduction per 8 J0s
+        // (16 accumulators); fewer ranges take the smallest tile holding them
+        if (nr <= 1)
+            k_quad_rows<1><<<it.items, kRowThreads, 0, s>>>(ku, C, ranges, nr, fd, it, part);
+        else if (nr <= 2)
+            k_quad_rows<2><<<it.items, kRowThreads, 0, s>>>(ku, C, ranges, nr, fd, it, part);
+        else if (nr <= 4)
+            k_quad_rows<4><<<it.items, kRowThreads, 0, s>>>(ku, C, ranges, nr, fd, it, part);
+        else
+            k_quad_rows<8><<<(unsigned)it.items * ((nr + 7) / 8), kRowThreads, 0, s>>>(ku, C, ranges, nr, fd, it, part);
+    }
+    k_rows_finish<<<(unsigned)(((long long)nf * nr + 127) / 128), 128, 0, s>>>(part, C, ranges, nf, nr, fd, it, G);
+}
+
+int rows_item_size(long long wavenumbers, int nr) {
+    // about 16 blocks per SM of 148 over the launch's (item, range tile) blocks,
+    // between 2 wavenumbers a thread (a single response: latency) and 64 (the
+    // reduction, ~200 instructions a thread, is then under 1% of 64 x 8 J0s)
+    const long long tiles = nr <= 8 ? 1 : (nr + 7) / 8;
+    long long kc = wavenumbers * tiles / (148 * 16);
+    kc = (kc + kRowThreads - 1) / kRowThreads * kRowThreads;
+    return (int)std::min<long long>(std::max<long long>(kc, 2 * kRowThreads), 64 * kRowThreads);
 }
 
 // ------------------------------------------------------------ bank pack --

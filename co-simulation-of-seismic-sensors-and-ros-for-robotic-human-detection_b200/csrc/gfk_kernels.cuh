@@ -29,6 +29,18 @@ struct PropQueue {
     int items, runs;
 };
 
+// The wavenumbers of rows whose grids differ, cut into items of kc (a multiple
+// of 128) consecutive ones: item i (of the launch) is the (i - begin[f] + item0)-th
+// of row f = row[i] - row0, and row f's items are begin[f] - item0 to
+// begin[f + 1] - item0. With null tables the launch has one row of `items` items.
+// row and begin point at the launch's first item and first row.
+struct RowItems {
+    const int* row;
+    const int* begin;
+    int row0, item0, items, kc;
+};
+int rows_item_size(long long wavenumbers, int nr);
+
 // rem[fd[f].off + i - 1] = k_i u(k_i, f) - C_f for i = 1..nk, k_i = i dk.
 // `variant` picks one of prop_variant_count() launch shapes of the Dunkin
 // kernel; the persistent ones (prop_variant_persistent) take their items from
@@ -87,9 +99,13 @@ int quad_gemm_splits(int nf, int nk, int nr);
 void launch_quad_finish(cudaStream_t s, const cd* part, int splits, const cd* C, const double* ranges, int nf,
                         int nr, double dk, cd* G);
 
-// Per-frequency grids: the same sum with J0 evaluated in the loop.
-void launch_quad_ragged(cudaStream_t s, const cd* rem, const cd* C, const double* ranges, int nf, int nr,
-                        const FreqDesc* fd, cd* G);
+// Per-frequency grids: ku[fd[f].off + i - 1] = k_i u(k_i, f) over items, with
+// the static coefficients C; then the sum of ku - C with J0 evaluated in the
+// loop; part holds items x nr.
+void launch_prop_rows(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, int nf,
+                      const cd* wc2, cd* C, int formulation, cd* ku, int* status, const RowItems& it);
+void launch_quad_rows(cudaStream_t s, const cd* ku, const cd* C, const double* ranges, int nf, int nr,
+                      const FreqDesc* fd, const RowItems& it, cd* part, cd* G);
 
 void launch_bank_pack(cudaStream_t s, const cd* G, int nf, int nr, int first_bin, int bins, float* payload);
 

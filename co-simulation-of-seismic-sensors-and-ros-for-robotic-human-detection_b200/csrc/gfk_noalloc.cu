@@ -42,6 +42,8 @@ constexpr size_t kOffRanges = kOffScalars + 256;                                
 constexpr size_t kOffG = kOffRanges + size_t(GFK_NOALLOC_MAX_RANGES) * 8;          // cd[nr]
 constexpr size_t kOffRem = kOffG + size_t(GFK_NOALLOC_MAX_RANGES) * 16;            // cd[nk]
 static_assert(kOffRem + size_t(GFK_NOALLOC_MAX_SAMPLES) * 16 <= kNoallocScratchBytes, "scratch too small");
+static_assert(kOffRem + (size_t(GFK_NOALLOC_MAX_SAMPLES) + GFK_NOALLOC_MAX_RANGES) * 16 <= kNoallocScratchBytes,
+              "no room for one partial sum per range");
 static_assert(64 * sizeof(gfk::LayerP) <= kOffLayersC, "layer block too small");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocScratchBytes];
@@ -193,9 +195,14 @@ extern "C" int gfk_vertical_displacement_multi_noalloc(const gfk_medium* m, cons
     if (e != cudaSuccess) return GFK_ECUDA;
     const int form = s->formulation;
     gfk::launch_layer_consts(strm, d_lp, d_medium, d_row, 1, s->omega_imag, form, d_lc, d_wc2);
-    gfk::launch_static(strm, d_lc, d_medium, d_row, d_wc2, 1, form, d_C, d_status);
-    gfk::launch_prop(strm, d_lc, d_medium, d_row, d_wc2, 1, g.samples, d_C, form, d_rem, d_status);
-    gfk::launch_quad_ragged(strm, d_rem, d_C, d_r, 1, nr, d_row, d_G);
+    // the partial sums of as many items as the rest of the array holds
+    const size_t part_off = kOffRem + (size_t)g.samples * 16;
+    const size_t fit = (kNoallocScratchBytes - part_off) / ((size_t)nr * 16);
+    int kc = gfk::rows_item_size(g.samples, nr);
+    while ((size_t)((g.samples + kc - 1) / kc) > fit) kc *= 2;
+    const gfk::RowItems it{nullptr, nullptr, 0, 0, (g.samples + kc - 1) / kc, kc};
+    gfk::launch_prop_rows(strm, d_lc, d_medium, d_row, 1, d_wc2, d_C, form, d_rem, d_status, it);
+    gfk::launch_quad_rows(strm, d_rem, d_C, d_r, 1, nr, d_row, it, reinterpret_cast<cd*>(base + part_off), d_G);
     ok(cudaGetLastError());
     int flags = 0;
     ok(cudaMemcpyAsync(out, d_G, sizeof(cd) * nr, cudaMemcpyDeviceToHost, strm));

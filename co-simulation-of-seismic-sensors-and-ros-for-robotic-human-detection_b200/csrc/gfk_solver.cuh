@@ -409,6 +409,57 @@ __device__ __forceinline__ bool m4_solve(M4 m, cd x[4], cd out[4]) {
     return true;
 }
 
+// The inverse as fk.go:195-213 takes it: one solve per unit vector. The four
+// solves share the matrix, so its elimination runs once for the four
+// right-hand sides: the operations on each are m4_solve's, in its order.
+__device__ __forceinline__ bool m4_inverse(M4 m, M4& x) {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) x.a[i][j] = mk(i == j ? 1.0 : 0.0);
+#pragma unroll
+    for (int col = 0; col < 4; col++) {
+        double best = 0.0;
+        int brow = col;
+#pragma unroll
+        for (int r = col; r < 4; r++) {
+            const double v = cabs_(m.a[r][col]);
+            if (v > best) { best = v; brow = r; }
+        }
+        if (best == 0.0) return false;
+#pragma unroll
+        for (int r = col + 1; r < 4; r++) {
+            if (r == brow) {
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    cd t = m.a[col][c]; m.a[col][c] = m.a[r][c]; m.a[r][c] = t;
+                    t = x.a[col][c]; x.a[col][c] = x.a[r][c]; x.a[r][c] = t;
+                }
+            }
+        }
+        const cd p = m.a[col][col];
+#pragma unroll
+        for (int r = col + 1; r < 4; r++) {
+            const cd f = m.a[r][col] / p;
+            if (f.re == 0.0 && f.im == 0.0) continue;
+#pragma unroll
+            for (int c = col; c < 4; c++) m.a[r][c] -= f * m.a[col][c];
+#pragma unroll
+            for (int c = 0; c < 4; c++) x.a[r][c] -= f * x.a[col][c];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int i = 3; i >= 0; i--) {
+            cd s = x.a[i][c];
+#pragma unroll
+            for (int j = i + 1; j < 4; j++) s -= m.a[i][j] * x.a[j][c];
+            x.a[i][c] = s / m.a[i][i];
+        }
+    return true;
+}
+
 // props.eigen (fk.go:138-168): columns (P down, SV down, P up, SV up).
 __device__ __forceinline__ void eigen4(const LayerC& L, double k, double omega, double mu_ref, cd lam[4], M4& e) {
     const cd alpha = L.c[0], beta = L.c[1], mu = L.c[2];
@@ -452,15 +503,7 @@ __device__ __forceinline__ cd direct_u(const LayerC* L, int n, double omega, dou
 #pragma unroll
         for (int i = 0; i < 4; i++) d[i] = cexp_((lam[i] - max_re) * zeta);
         M4 inv;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            cd ej[4] = {mk(0), mk(0), mk(0), mk(0)};
-            ej[j] = mk(1.0);
-            cd col[4];
-            if (!m4_solve(e, ej, col)) { ok = false; return mk(0.0); }
-#pragma unroll
-            for (int i = 0; i < 4; i++) inv.a[i][j] = col[i];
-        }
+        if (!m4_inverse(e, inv)) { ok = false; return mk(0.0); }
         // p = (e d) inv; total = p total
         M4 p;
 #pragma unroll
