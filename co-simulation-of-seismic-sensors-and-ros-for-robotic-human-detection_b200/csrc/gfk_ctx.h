@@ -15,19 +15,21 @@ struct gfk_net;
 struct gfk_bank_dev;
 
 // The Hankel weights of a shared-grid wavenumber sum (the tensor-core sum's
-// int8 digit planes, or the plain sum's FP64 table). They depend only on the
+// int8 digit planes, the plain sum's FP64 table, or the few-range sum's table
+// followed by its panel weights). They depend only on the
 // grid and the ranges, so plans with the same ones share one device copy; it
 // is freed, ordered on the context's stream, when its last holder lets go.
 struct gfk_weights {
+    enum Kind { kTable, kDigits, kFused };
     gfk_ctx* ctx = nullptr;
-    bool tc = false;
+    Kind kind = kTable;
     int n = 0;         // wavenumbers
     double dk = 0.0;   // wavenumber step
     std::vector<double> ranges;
     void* d = nullptr;
     bool built = false;  // its build has been enqueued on the context's stream
-    bool same(bool tc_, int n_, double dk_, const double* r, int nr) const {
-        return tc == tc_ && n == n_ && dk == dk_ && (int)ranges.size() == nr &&
+    bool same(Kind kind_, int n_, double dk_, const double* r, int nr) const {
+        return kind == kind_ && n == n_ && dk == dk_ && (int)ranges.size() == nr &&
                std::equal(ranges.begin(), ranges.end(), r);
     }
     ~gfk_weights();
@@ -53,6 +55,7 @@ struct gfk_ctx {
         int Mp, Np, Kp, variant;
     };
     std::vector<TunedTc> tuned_tc;
+    double* panels = nullptr;  // the panel interpolation table (gfk_panel.cuh), built by gfk_open
     // the most recent plan's Hankel weights, kept for the next plan
     std::shared_ptr<gfk_weights> weights;
 };

@@ -12,6 +12,7 @@
 #include "../../include/gfk.h"
 #include "gfk_ctx.h"
 #include "gfk_kernels.cuh"
+#include "gfk_panel.cuh"
 
 
 
@@ -291,16 +292,16 @@ int dalloc(gfk_ctx* ctx, T** ptr, size_t count) {
 
 // The plan's Hankel weights: the context's cached copy when the grid and the
 // ranges match, else a new device buffer that becomes the cached one.
-int plan_weights(gfk_plan* p, bool tc, int n, double dk, size_t bytes) {
+int plan_weights(gfk_plan* p, gfk_weights::Kind kind, int n, double dk, size_t bytes) {
     gfk_ctx* ctx = p->ctx;
     const int nr = (int)p->ranges.size();
-    if (ctx->weights && ctx->weights->same(tc, n, dk, p->ranges.data(), nr)) {
+    if (ctx->weights && ctx->weights->same(kind, n, dk, p->ranges.data(), nr)) {
         p->wts = ctx->weights;
         return GFK_OK;
     }
     auto w = std::make_shared<gfk_weights>();
     w->ctx = ctx;
-    w->tc = tc;
+    w->kind = kind;
     w->n = n;
     w->dk = dk;
     w->ranges = p->ranges;
@@ -599,7 +600,7 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         int max_cnf = 0;
         for (size_t c = 0; c + 1 < p->chunk_begin.size(); c++)
             max_cnf = std::max(max_cnf, p->chunk_begin[c + 1] - p->chunk_begin[c]);
-        const int nkb = (g_n + 127) / 128;
+        const int nkb = (g_n + 1023) / 1024;
         if (!st) st = dalloc(ctx, &p->d_partial, (size_t)max_cnf * nkb * nr);
     } else if (!st) {
         st = dalloc(ctx, &p->d_rem, (size_t)std::max<int64_t>(cap, 1));
@@ -610,7 +611,9 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         if (!st) st = dalloc(ctx, &p->d_ksum, (size_t)max_items * nr);
     }
     if (!st && p->shared && !p->tc) {
-        if (!(st = plan_weights(p, false, g_n, g_kmax / g_n, sizeof(double) * (size_t)g_n * nr)))
+        const size_t count = (size_t)g_n * nr + (p->fused ? gfk::panel_weight_count(g_n, nr) : 0);
+        if (!(st = plan_weights(p, p->fused ? gfk_weights::kFused : gfk_weights::kTable, g_n, g_kmax / g_n,
+                                sizeof(double) * count)))
             p->d_W = static_cast<double*>(p->wts->d);
     }
     if (!st && p->tc) {
@@ -625,7 +628,7 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         // past a chunk's 2 cnf are computed by the sum but never stored, so
         // the planes need no clearing
         st = dalloc(ctx, &p->d_A, (size_t)4 * p->Mp * p->Kp);
-        if (!st && !(st = plan_weights(p, true, g_n, g_kmax / g_n, (size_t)4 * p->Np * p->Kp)))
+        if (!st && !(st = plan_weights(p, gfk_weights::kDigits, g_n, g_kmax / g_n, (size_t)4 * p->Np * p->Kp)))
             p->d_B = static_cast<int8_t*>(p->wts->d);
         if (!st) st = dalloc(ctx, &p->d_rowexp, (size_t)p->Mp);
         if (!st) st = dalloc(ctx, &p->d_rowmax, (size_t)3 * max_cnf);  // row maxima, then finished-block counts
@@ -716,7 +719,7 @@ int tune_prop(gfk_plan* p) {
             cudaMemsetAsync(p->d_queue, 0, sizeof(unsigned int), s);
             cudaEventRecord(a, s);
             gfk::launch_prop(s, p->d_lc, p->d_media, p->d_fd + fb, p->d_wc2 + fb, win, cmax, p->d_C + fb,
-                             GFK_DUNKIN, p->d_rem, p->d_status + fb, v, p->tc ? &so : nullptr, p->d_queue);
+                             GFK_DUNKIN, ctx->panels, p->d_rem, p->d_status + fb, v, p->tc ? &so : nullptr, p->d_queue);
             cudaEventRecord(b, s);
             ctx->launches++;
             cudaError_t e = cudaEventSynchronize(b);
@@ -826,6 +829,10 @@ int plan_enqueue(gfk_plan* p, bool timed) {
         else
             gfk::launch_j0_table(s, p->d_ranges, p->nr, p->g_n, p->g_kmax / p->g_n, p->d_W);
         ctx->launches++;
+        if (p->fused) {
+            gfk::launch_panel_weights(s, p->d_W, ctx->panels, p->g_n, p->nr, p->d_W + (size_t)p->g_n * p->nr);
+            ctx->launches++;
+        }
         p->wts->built = true;
     }
     if (timed && (st = end_seg(p, seg))) return st;
@@ -840,7 +847,8 @@ int plan_enqueue(gfk_plan* p, bool timed) {
         if (p->fused) {
             if (timed && (st = begin_seg(p, 0, &seg))) return st;
             gfk::launch_prop_fused(s, p->d_lc, p->d_media, p->d_fd + fb, p->d_wc2 + fb, cnf, p->g_n, p->d_C + fb,
-                                   p->d_W, p->d_ranges, p->nr, p->d_partial, p->d_status + fb,
+                                   ctx->panels, p->d_W, p->d_W + (size_t)p->g_n * p->nr, p->d_ranges, p->nr,
+                                   p->d_partial, p->d_status + fb,
                                    p->d_G + (size_t)fb * p->nr);
             if (timed && (st = end_seg(p, seg))) return st;
             ctx->launches += 2;
@@ -850,8 +858,8 @@ int plan_enqueue(gfk_plan* p, bool timed) {
         if (!p->shared) {
             const gfk::RowItems it = row_items(p, fb, cnf);
             if (timed && (st = begin_seg(p, 0, &seg))) return st;
-            gfk::launch_prop_rows(s, p->d_lc, p->d_media, p->d_fd + fb, cnf, p->d_wc2 + fb, p->d_C + fb, form, p->d_rem,
-                                  p->d_status + fb, it);
+            gfk::launch_prop_rows(s, p->d_lc, p->d_media, p->d_fd + fb, cnf, p->d_wc2 + fb, p->d_C + fb, form, ctx->panels,
+                                  p->d_rem, p->d_status + fb, it);
             if (timed && (st = end_seg(p, seg))) return st;
             if (timed && (st = begin_seg(p, 1, &seg))) return st;
             gfk::launch_quad_rows(s, p->d_rem, p->d_C + fb, p->d_ranges, cnf, p->nr, p->d_fd + fb, it, p->d_ksum,
@@ -867,7 +875,7 @@ int plan_enqueue(gfk_plan* p, bool timed) {
         if (gfk::prop_variant_persistent(p->prop_variant))
             GFK_CUDA(ctx, cudaMemsetAsync(p->d_queue, 0, sizeof(unsigned int), s));
         if (timed && (st = begin_seg(p, 0, &seg))) return st;
-        gfk::launch_prop(s, p->d_lc, p->d_media, p->d_fd + fb, p->d_wc2 + fb, cnf, cmax, p->d_C + fb, form, p->d_rem,
+        gfk::launch_prop(s, p->d_lc, p->d_media, p->d_fd + fb, p->d_wc2 + fb, cnf, cmax, p->d_C + fb, form, ctx->panels, p->d_rem,
                          p->d_status + fb, std::max(p->prop_variant, 0), p->tc ? &so : nullptr, p->d_queue);
         if (timed && (st = end_seg(p, seg))) return st;
         if (timed && (st = begin_seg(p, 1, &seg))) return st;
@@ -1006,6 +1014,14 @@ int gfk_open(int device, gfk_ctx** out) {
         uint64_t thr = UINT64_MAX;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
+    const std::vector<double> tab = gfk::panel_table();
+    if (cudaMallocAsync((void**)&c->panels, sizeof(double) * tab.size(), c->stream) != cudaSuccess ||
+        cudaMemcpyAsync(c->panels, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, c->stream) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(c->stream) != cudaSuccess) {
+        gfk_close(c);
+        return GFK_ECUDA;
+    }
     *out = c;
     return GFK_OK;
 }
@@ -1023,6 +1039,7 @@ int gfk_close(gfk_ctx* ctx) {
     }
     ctx->plans.clear();
     ctx->weights.reset();
+    if (ctx->panels) cudaFreeAsync(ctx->panels, ctx->stream);
     gfk_release_surrogates(ctx);
     gfk_release_banks(ctx);
     if (ctx->copy_stream) {

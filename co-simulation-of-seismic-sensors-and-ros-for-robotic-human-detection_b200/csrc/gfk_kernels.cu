@@ -13,6 +13,8 @@
 //                   (internal/bank/format.go:185-193)
 #include "gfk_kernels.cuh"
 #include "gfk_j0.cuh"
+#include "gfk_panel.cuh"
+
 
 #include <algorithm>
 #include <atomic>
@@ -138,84 +140,278 @@ void launch_static(cudaStream_t s, const LayerC* lc, const MediumP* media, const
 
 // ------------------------------------------------------------ propagator --
 //
-// The work item is (row f, run): one thread per (f, k) (ILP = 1) or per
-// (f, k, k + THREADS) pair (ILP = 2, two wavenumbers in lockstep), SWEEPS
-// times over consecutive stretches of THREADS x ILP wavenumbers; a row has
-// `runs` items. k_prop serves one item per block (blockIdx = (run, f));
-// k_prop_q is persistent: each resident block takes items from a device
-// queue in row order until none are left. The row's layer constants are
-// staged in shared memory. Launch shapes are template parameters; the plan
-// times them once and keeps the fastest.
+// The work item is (row f, run): 8 panels of 128 wavenumbers per 128 threads
+// (gfk_panel.cuh). Pass 0 solves the 16 first nodes of every panel, one per
+// thread, a half-warp per panel, which tests its coefficients by shuffles;
+// pass 1 the other 16 nodes of the panels that may be served by 32; the passes
+// after that every wavenumber of the remaining panels. One loop holds the
+// three, so the solve is compiled once. The interpolation of the accepted
+// panels is a product of a fixed 128 x 16 (or 32) matrix and the node values,
+// 4 panels (re, im) wide, on the FP64 tensor path: as many FP64-pipe cycles as
+// FMAs, an eighth of the issue slots and no operand traffic (the matrix
+// fragments come from L1).
+//
+// k_prop serves one item per block (blockIdx = (run, f)); k_prop_q is
+// persistent: each resident block takes items from a device queue in row order
+// until none are left. The row's layer constants are staged in shared memory.
+// Launch shapes are template parameters; the plan times them once and keeps
+// the fastest. The direct formulation solves every wavenumber: its parity with
+// the reference includes the digits its eigenbasis loses.
+
+constexpr int kNodeStride = kPanelN + 4;  // of the node values in shared memory: conflict-free B fragments
 
 // Shared memory of one propagator block.
 template <int THREADS, bool SLICE>
 struct PropSmem {
     LayerC lc[kMaxLayers];
-    cd tile[SLICE ? THREADS * 8 : 1];
+    union {
+        cd tile[SLICE ? THREADS * 8 : 1];
+        cd nodes[THREADS / 16 * kNodeStride];
+    };
+    unsigned char mode[THREADS / 16];
     int last, item;
+    __device__ PropSmem() {}
 };
 
+// FP64 tensor-path product D = A B + D, m8n8k4: lane t holds A[t/4][t%4],
+// B[t%4][t/4] and D[t/4][2(t%4) + {0,1}]. Not volatile: the result is used, and
+// the compiler may move the next step's fragment loads ahead of these MMAs.
+__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c0), "+d"(c1)
+        : "d"(a), "d"(b));
+}
+
+// The three last (and, MID, three middle) Chebyshev coefficients of the warp's
+// two panels, lane 16 p + j holding node j of panel p in v[] (one value per 16
+// nodes): an 8 x 16 T times 16 T x 4 product on the FP64 tensor path, whose B
+// fragments are shuffled out of the lanes (half the shuffles of a reduction
+// tree per coefficient, and 4 T instructions for the sums). rows: the table's
+// coefficient rows as A fragments. Returns this lane's panel's largest
+// |part| of a last coefficient, and of a middle one in mid; NaN where one is.
+template <int T, bool MID>
+__device__ __forceinline__ double panel_tail(const double* __restrict__ rows, const cd (&v)[T], double& mid) {
+    const int lane = threadIdx.x & 31;
+    const int src = ((lane >> 3) & 1) * 16 + (lane & 3);  // column lane/4: panel, part
+    const bool im = (lane >> 2) & 1;
+    double c0 = 0.0, c1 = 0.0;
+#pragma unroll
+    for (int t = 0; t < T; t++)
+#pragma unroll
+        for (int kk = 0; kk < 4; kk++) {
+            const double re = __shfl_sync(0xffffffffu, v[t].re, src + 4 * kk);
+            const double iv = __shfl_sync(0xffffffffu, v[t].im, src + 4 * kk);
+            dmma(c0, c1, rows[(4 * t + kk) * 32 + lane], im ? iv : re);
+        }
+    // lane 4 row + p (p < 2) holds (re, im) of coefficient `row` of panel p
+    double m = fmax(fabs(c0), fabs(c1));
+    if (isnan(c0) || isnan(c1)) m = INFINITY;
+    const int p = lane >> 4;
+    mid = 0.0;
+    if (MID)
+        mid = fmax(__shfl_sync(0xffffffffu, m, 12 + p),
+                   fmax(__shfl_sync(0xffffffffu, m, 16 + p), __shfl_sync(0xffffffffu, m, 20 + p)));
+    return fmax(__shfl_sync(0xffffffffu, m, p), fmax(__shfl_sync(0xffffffffu, m, 4 + p), __shfl_sync(0xffffffffu, m, 8 + p)));
+}
+
+// The largest of the half-warp's non-negative values, to 2^-20 (its high word).
+__device__ __forceinline__ double half_max(double v) {
+    int h = __double2hiint(v);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) h = max(h, __shfl_xor_sync(0xffffffffu, h, o));
+    return __hiloint2double(h, 0);
+}
+
+// The panels of one item, [base, lim) of row f's n wavenumbers (lim a panel's
+// end or n). NR = 0: the integrand goes to row[]; NR > 0: each value is added
+// to acc times the range's weights, W[wavenumber][nr] or, for a whole panel,
+// Wp[panel][48][nr] (the weights carried over to its 16 or 32 nodes). SUB: the
+// values are k u - c, else k u.
+template <int THREADS, int NR, bool SUB, class SMEM>
+__device__ __forceinline__ void panel_item(const double* __restrict__ tab, SMEM& sm, int nl, double mu_ref, cd w2,
+                                           cd c, double d, int n, int base, int lim, cd* __restrict__ row,
+                                           const double* __restrict__ W, const double* __restrict__ Wp, int nr,
+                                           double* acc, double& mre, double& mim, int& bad) {
+    constexpr int PANELS = THREADS / 16;
+    const int tid = threadIdx.x, hp = tid >> 4, hj = tid & 15;
+    const int pa = base + kPanel * hp;
+    const bool use = pa < lim && n - pa >= kPanelLeast;
+    const double cabs1 = SUB ? cnorm1(c) : 0.0;
+    cd first = mk(0.0);
+    double big = 0.0;
+    bool more = false;
+    int mode = 0;
+    unsigned direct = 0;
+#pragma unroll 1
+    for (int pass = 0;; pass++) {
+        double x;  // wavenumber / d
+        bool live;
+        int i = 0;
+        if (pass < 2) {
+            live = pass == 0 ? use : more;
+            x = fma(64.0, tab[kPtX + pass * kPanelE + hj], (double)pa + 64.5);
+        } else {
+            if (direct == 0) break;
+            i = base + kPanel * (__ffs(direct) - 1) + (tid & (kPanel - 1)) + 1;
+            if constexpr (THREADS > kPanel) {  // the upper threads take the next panel
+                const unsigned rest = direct & (direct - 1);
+                if (tid >= kPanel) i = rest ? base + kPanel * (__ffs(rest) - 1) + (tid & (kPanel - 1)) + 1 : n + 1;
+                direct = rest;
+            }
+            direct &= direct - 1;
+            live = i <= n;
+            x = (double)i;
+        }
+        cd r = mk(0.0);
+        if (live) {
+            const double k = x * d;
+            r = k * dunkin_u(sm.lc, nl, w2, k, mu_ref);
+            if (SUB) r -= c;
+        }
+        if (pass == 0) {
+            first = r;
+            big = half_max(cnorm1(r));
+            const cd v[1] = {r};
+            double mid;
+            const double tail = panel_tail<1, true>(tab + kPtRowsE, v, mid);
+            const double scale = cabs1 + big;
+            mode = use && tail <= kPanelTol * scale;
+            // decay per 6 orders, q = tail/mid; at order 31: tail q^(16/6) <= 10 tol scale
+            const float s = (float)(1.0 / scale), tl = (float)tail * s, q = tl / ((float)mid * s);
+            const float room = (float)(10.0 * kPanelTol) / tl, q2 = q * q, q4 = q2 * q2;
+            more = use && !mode && q < 1.0f && q4 * q4 <= room * room * room;
+            if (NR == 0) sm.nodes[hp * kNodeStride + hj] = r;
+        } else if (pass == 1) {
+            if (__any_sync(0xffffffffu, more)) {
+                const double m2 = half_max(cnorm1(r));
+                const cd v[2] = {first, r};
+                double none;
+                const double tail = panel_tail<2, false>(tab + kPtRowsN, v, none);
+                if (more && tail <= kPanelTol * (cabs1 + fmax(big, m2))) mode = 2;
+            }
+            if constexpr (NR > 0) {
+                if (mode) {
+                    const double* w = Wp + ((size_t)(pa / kPanel) * 48 + (mode == 1 ? 0 : kPanelE) + hj) * nr;
+#pragma unroll
+                    for (int q = 0; q < NR; q++)
+                        if (q < nr) {
+                            acc[2 * q] = fma(first.re, w[q], acc[2 * q]);
+                            acc[2 * q + 1] = fma(first.im, w[q], acc[2 * q + 1]);
+                            if (mode == 2) {
+                                const double w1 = w[kPanelE * nr + q];
+                                acc[2 * q] = fma(r.re, w1, acc[2 * q]);
+                                acc[2 * q + 1] = fma(r.im, w1, acc[2 * q + 1]);
+                            }
+                        }
+                }
+            } else {
+                sm.nodes[hp * kNodeStride + kPanelE + hj] = r;
+            }
+            if (hj == 0) sm.mode[hp] = (unsigned char)mode;
+            __syncthreads();
+#pragma unroll
+            for (int p = 0; p < PANELS; p++)
+                if (sm.mode[p] == 0 && base + kPanel * p < lim) direct |= 1u << p;
+        } else if (live) {
+            if (!(isfinite(r.re) && isfinite(r.im))) { bad |= kStNonfinite; r = mk(0.0); }
+            if constexpr (NR > 0) {
+#pragma unroll
+                for (int q = 0; q < NR; q++) {
+                    const double w = q < nr ? W[(size_t)(i - 1) * nr + q] : 0.0;
+                    acc[2 * q] = fma(r.re, w, acc[2 * q]);
+                    acc[2 * q + 1] = fma(r.im, w, acc[2 * q + 1]);
+                }
+            } else {
+                row[i - 1] = r;
+                mre = fmax(mre, fabs(r.re));
+                mim = fmax(mim, fabs(r.im));
+            }
+        }
+    }
+    if constexpr (NR == 0) {
+        // warp w holds points 32 w' .. + 31 (w' = w mod 4) of 4 panels at a time:
+        // C fragment row = point, columns 2 (panel) + part
+        const int lane = tid & 31, wq = (tid >> 5) & 3;
+#pragma unroll 1
+        for (int g = (tid >> 7) * 4; g < PANELS; g += THREADS / kPanel * 4) {
+            const int bm = sm.mode[g + (lane >> 3)];
+            const bool any1 = __any_sync(0xffffffffu, bm == 1), any2 = __any_sync(0xffffffffu, bm == 2);
+            if (!any1 && !any2) continue;
+            const double* v = reinterpret_cast<const double*>(sm.nodes + (g + (lane >> 3)) * kNodeStride + (lane & 3)) +
+                              ((lane >> 2) & 1);
+            double y[4][2];
+#pragma unroll
+            for (int m = 0; m < 4; m++) y[m][0] = y[m][1] = 0.0;
+            if (any1) {
+#pragma unroll
+                for (int kk = 0; kk < kPanelE / 4; kk++) {
+                    const double bv = bm == 1 ? v[8 * kk] : 0.0;
+#pragma unroll
+                    for (int m = 0; m < 4; m++)
+                        dmma(y[m][0], y[m][1], tab[kPtFragE + ((4 * wq + m) * (kPanelE / 4) + kk) * 32 + lane], bv);
+                }
+            }
+            if (any2) {
+#pragma unroll
+                for (int kk = 0; kk < kPanelN / 4; kk++) {
+                    const double bv = bm == 2 ? v[8 * kk] : 0.0;
+#pragma unroll
+                    for (int m = 0; m < 4; m++)
+                        dmma(y[m][0], y[m][1], tab[kPtFragN + ((4 * wq + m) * (kPanelN / 4) + kk) * 32 + lane], bv);
+                }
+            }
+            const int p = g + (lane & 3);
+            if (sm.mode[p])
+#pragma unroll
+                for (int m = 0; m < 4; m++) {
+                    const int at = base + kPanel * p + (4 * wq + m) * 8 + (lane >> 2);
+                    if (at < n) {
+                        row[at] = mk(y[m][0], y[m][1]);
+                        mre = fmax(mre, fabs(y[m][0]));
+                        mim = fmax(mim, fabs(y[m][1]));
+                    }
+                }
+        }
+    }
+}
+
 // `stage`: the block's staged layer constants are not row f's (uniform).
-template <int FORM, int THREADS, int ILP, int SWEEPS, bool SLICE>
+template <int FORM, int THREADS, bool SLICE>
 __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const MediumP* __restrict__ media,
                                           const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2,
-                                          const cd* __restrict__ C, cd* __restrict__ rem, int* __restrict__ status,
-                                          const SliceOut& so, int f, int run, int runs, bool stage,
-                                          PropSmem<THREADS, SLICE>& sm) {
-    LayerC* const s_lc = sm.lc;
+                                          const cd* __restrict__ C, const double* __restrict__ tab,
+                                          cd* __restrict__ rem, int* __restrict__ status, const SliceOut& so, int f,
+                                          int run, int runs, bool stage, PropSmem<THREADS, SLICE>& sm) {
     const FreqDesc fdesc = fd[f];
     const MediumP med = media[fdesc.soil];
     const int nl = med.count;
     const double mu_ref = med.mu_ref;
     if (stage) {
-        for (int l = threadIdx.x; l < nl; l += blockDim.x) s_lc[l] = lc[fdesc.lc_off + l];
+        for (int l = threadIdx.x; l < nl; l += blockDim.x) sm.lc[l] = lc[fdesc.lc_off + l];
         __syncthreads();
     }
     const int n = fdesc.kfar > 0 ? fdesc.nk : 0;
     const double d = fdesc.dk;
     const cd c = C ? C[f] : mk(0.0);
-    const cd w2 = wc2[f];
     cd* row = rem + fdesc.off;
     int bad = 0;
     double mre = 0.0, mim = 0.0;
-#pragma unroll 1
-    for (int sw = 0; sw < SWEEPS; sw++) {
-        const int i0 = (run * SWEEPS + sw) * (THREADS * ILP) + threadIdx.x + 1;
-        if (i0 > n) break;
-        if (FORM == 0) {
+    if constexpr (FORM == 0) {
+        const int i = run * THREADS + threadIdx.x + 1;
+        if (i <= n) {
             bool ok;
-            const double k = (double)i0 * d;
-            cd u = direct_u(s_lc, nl, kTwoPi * fdesc.freq, k, mu_ref, ok);
+            const double k = (double)i * d;
+            cd u = direct_u(sm.lc, nl, kTwoPi * fdesc.freq, k, mu_ref, ok);
             if (!ok) bad |= kStSingular;
             cd r = k * u - c;
             if (!finite_cd(r)) { bad |= kStNonfinite; r = mk(0.0); }
-            row[i0 - 1] = r;
-            mre = fmax(mre, fabs(r.re)); mim = fmax(mim, fabs(r.im));
-        } else if (ILP == 1) {
-            const double k = (double)i0 * d;
-            const cd u = dunkin_u(s_lc, nl, w2, k, mu_ref);
-            cd r = k * u - c;
-            if (!finite_cd(r)) { bad |= kStNonfinite; r = mk(0.0); }
-            row[i0 - 1] = r;
-            mre = fmax(mre, fabs(r.re)); mim = fmax(mim, fabs(r.im));
-        } else {
-            const int i1 = i0 + THREADS;
-            const bool has1 = i1 <= n;
-            const double k0 = (double)i0 * d;
-            const double k1 = has1 ? (double)i1 * d : k0;
-            cd u0, u1;
-            dunkin_u2(s_lc, nl, w2, k0, k1, mu_ref, u0, u1);
-            cd r0 = k0 * u0 - c;
-            if (!finite_cd(r0)) { bad |= kStNonfinite; r0 = mk(0.0); }
-            row[i0 - 1] = r0;
-            mre = fmax(mre, fabs(r0.re)); mim = fmax(mim, fabs(r0.im));
-            if (has1) {
-                cd r1 = k1 * u1 - c;
-                if (!finite_cd(r1)) { bad |= kStNonfinite; r1 = mk(0.0); }
-                row[i1 - 1] = r1;
-                mre = fmax(mre, fabs(r1.re)); mim = fmax(mim, fabs(r1.im));
-            }
+            row[i - 1] = r;
+            mre = fabs(r.re);
+            mim = fabs(r.im);
         }
+    } else {
+        panel_item<THREADS, 0, true>(tab, sm, nl, mu_ref, wc2[f], c, d, n, run * THREADS * 8, n, row, nullptr, nullptr,
+                                     0, nullptr, mre, mim, bad);
     }
     if (bad) atomicOr(status + f, bad);
     if constexpr (SLICE) {
@@ -258,15 +454,16 @@ __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const M
     }
 }
 
-template <int FORM, int THREADS, int MINB, int ILP, int SWEEPS, bool SLICE>
+template <int FORM, int THREADS, int MINB, bool SLICE>
 __global__ __launch_bounds__(THREADS, MINB) void k_prop(const LayerC* __restrict__ lc,
                                                        const MediumP* __restrict__ media,
                                                        const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2,
-                                                       const cd* __restrict__ C, cd* __restrict__ rem,
-                                                       int* __restrict__ status, SliceOut so, PropQueue) {
+                                                       const cd* __restrict__ C, const double* __restrict__ tab,
+                                                       cd* __restrict__ rem, int* __restrict__ status, SliceOut so,
+                                                       PropQueue) {
     __shared__ PropSmem<THREADS, SLICE> sm;
-    prop_item<FORM, THREADS, ILP, SWEEPS, SLICE>(lc, media, fd, wc2, C, rem, status, so, blockIdx.y, blockIdx.x,
-                                                 gridDim.x, true, sm);
+    prop_item<FORM, THREADS, SLICE>(lc, media, fd, wc2, C, tab, rem, status, so, blockIdx.y, blockIdx.x, gridDim.x,
+                                    true, sm);
 }
 
 // Rows of uneven length: block (item, y) serves the y-th run of 128
@@ -276,13 +473,17 @@ __global__ __launch_bounds__(THREADS, MINB) void k_prop(const LayerC* __restrict
 // blocks past the last item: one solve is a serial chain (89 us alone in the
 // direct formulation), so the integrand is stored as k u and the sum takes
 // C off.
-template <int FORM>
+// Block (item, y): the y-th 128 wavenumbers (solved one by one) or 1024 (by
+// panels, PANEL) of the item.
+template <int FORM, bool PANEL>
 __global__ __launch_bounds__(128, FORM == 0 ? 1 : 5) void k_prop_rows(const LayerC* __restrict__ lc,
                                                                      const MediumP* __restrict__ media,
                                                                      const FreqDesc* __restrict__ fd, int nf,
                                                                      const cd* __restrict__ wc2, cd* __restrict__ C,
+                                                                     const double* __restrict__ tab,
                                                                      cd* __restrict__ ku, int* __restrict__ status,
                                                                      RowItems it) {
+    constexpr int RUN = PANEL ? 8 * kPanel : 128;
     __shared__ PropSmem<128, false> sm;
     const int item = blockIdx.x;
     if (item >= it.items) {
@@ -291,20 +492,49 @@ __global__ __launch_bounds__(128, FORM == 0 ? 1 : 5) void k_prop_rows(const Laye
         return;
     }
     const int f = it.row ? it.row[item] - it.row0 : 0;
-    const int run = (item - (it.begin ? it.begin[f] - it.item0 : 0)) * (it.kc / 128) + blockIdx.y;
-    if (run * 128 >= fd[f].nk) return;
-    prop_item<FORM, 128, 1, 1, false>(lc, media, fd, wc2, nullptr, ku, status, SliceOut{}, f, run, 0, true, sm);
+    const int first = (item - (it.begin ? it.begin[f] - it.item0 : 0)) * it.kc;
+    const FreqDesc fdesc = fd[f];
+    const int base = first + blockIdx.y * RUN, lim = min(first + it.kc, fdesc.nk);
+    if (base >= lim) return;
+    const MediumP med = media[fdesc.soil];
+    for (int l = threadIdx.x; l < med.count; l += 128) sm.lc[l] = lc[fdesc.lc_off + l];
+    __syncthreads();
+    cd* row = ku + fdesc.off;
+    int bad = 0;
+    if constexpr (PANEL) {
+        double mre = 0.0, mim = 0.0;
+        panel_item<128, 0, false>(tab, sm, med.count, med.mu_ref, wc2[f], mk(0.0), fdesc.dk, fdesc.nk, base, lim, row,
+                                  nullptr, nullptr, 0, nullptr, mre, mim, bad);
+    } else {
+        const int i = base + threadIdx.x + 1;
+        if (i <= lim) {
+            const double k = (double)i * fdesc.dk;
+            cd u;
+            if (FORM == 0) {
+                bool ok;
+                u = direct_u(sm.lc, med.count, kTwoPi * fdesc.freq, k, med.mu_ref, ok);
+                if (!ok) bad |= kStSingular;
+            } else {
+                u = dunkin_u(sm.lc, med.count, wc2[f], k, med.mu_ref);
+            }
+            cd r = k * u;
+            if (!finite_cd(r)) { bad |= kStNonfinite; r = mk(0.0); }
+            row[i - 1] = r;
+        }
+    }
+    if (bad) atomicOr(status + f, bad);
 }
 
 // Persistent: items (f, run) in row order from q.next (zero at launch), so a
 // row's items run together and the row is sliced while it is in L2. Blocks
 // never wait for one another; each leaves when the queue is empty.
-template <int FORM, int THREADS, int MINB, int ILP, int SWEEPS, bool SLICE>
+template <int FORM, int THREADS, int MINB, bool SLICE>
 __global__ __launch_bounds__(THREADS, MINB) void k_prop_q(const LayerC* __restrict__ lc,
                                                          const MediumP* __restrict__ media,
                                                          const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2,
-                                                         const cd* __restrict__ C, cd* __restrict__ rem,
-                                                         int* __restrict__ status, SliceOut so, PropQueue q) {
+                                                         const cd* __restrict__ C, const double* __restrict__ tab,
+                                                         cd* __restrict__ rem, int* __restrict__ status, SliceOut so,
+                                                         PropQueue q) {
     __shared__ PropSmem<THREADS, SLICE> sm;
     int cur = -1;
     for (;;) {
@@ -314,36 +544,32 @@ __global__ __launch_bounds__(THREADS, MINB) void k_prop_q(const LayerC* __restri
         const int item = sm.item;
         if (item >= q.items) return;
         const int f = item / q.runs, run = item - f * q.runs;
-        prop_item<FORM, THREADS, ILP, SWEEPS, SLICE>(lc, media, fd, wc2, C, rem, status, so, f, run, q.runs, f != cur,
-                                                     sm);
+        prop_item<FORM, THREADS, SLICE>(lc, media, fd, wc2, C, tab, rem, status, so, f, run, q.runs, f != cur, sm);
         cur = f;
     }
 }
 
 namespace {
-using PropFn = void (*)(const LayerC*, const MediumP*, const FreqDesc*, const cd*, const cd*, cd*, int*, SliceOut,
-                        PropQueue);
+using PropFn = void (*)(const LayerC*, const MediumP*, const FreqDesc*, const cd*, const cd*, const double*, cd*, int*,
+                        SliceOut, PropQueue);
 struct PropVariant {
     PropFn fn, fn_slice;  // without and with the fused slicing
-    int threads, minb, ilp, sweeps;
+    int threads, minb;
     bool persistent;  // k_prop_q: one block per resident slot, items from a queue
 };
-#define GFK_PROP_SHAPE(T, B, I, S) {k_prop<1, T, B, I, S, false>, k_prop<1, T, B, I, S, true>, T, B, I, S, false}
-#define GFK_PROP_QUEUE(T, B, I, S) {k_prop_q<1, T, B, I, S, false>, k_prop_q<1, T, B, I, S, true>, T, B, I, S, true}
+#define GFK_PROP_SHAPE(T, B) {k_prop<1, T, B, false>, k_prop<1, T, B, true>, T, B, false}
+#define GFK_PROP_QUEUE(T, B) {k_prop_q<1, T, B, false>, k_prop_q<1, T, B, true>, T, B, true}
 const PropVariant kDunkinVariants[] = {
-    GFK_PROP_SHAPE(128, 4, 1, 1),  // <= 128 registers, 16 warps/SM
-    GFK_PROP_SHAPE(128, 5, 1, 1),  // <= 96 registers, 20 warps/SM
-    GFK_PROP_SHAPE(128, 6, 1, 1),  // <= 80 registers, 24 warps/SM
-    GFK_PROP_SHAPE(128, 2, 2, 1),  // two wavenumbers in lockstep, 8 warps/SM
-    GFK_PROP_SHAPE(64, 4, 2, 1),
-    GFK_PROP_SHAPE(256, 2, 1, 1),
-    GFK_PROP_SHAPE(128, 5, 1, 4),  // four runs of 128 wavenumbers per block
-    GFK_PROP_SHAPE(128, 5, 1, 8),
-    GFK_PROP_SHAPE(128, 4, 1, 4),
-    GFK_PROP_SHAPE(128, 4, 1, 8),
-    GFK_PROP_QUEUE(128, 5, 1, 1),  // persistent, items of 128, 256 and 512 wavenumbers
-    GFK_PROP_QUEUE(128, 5, 1, 2),
-    GFK_PROP_QUEUE(128, 5, 1, 4),
+    GFK_PROP_SHAPE(128, 3),  // <= 168 registers, 12 warps/SM
+    GFK_PROP_SHAPE(128, 4),  // <= 128 registers
+    GFK_PROP_SHAPE(128, 5),  // <= 96 registers
+    GFK_PROP_SHAPE(128, 6),  // <= 80 registers
+    GFK_PROP_SHAPE(256, 2),  // 16 panels per item
+    GFK_PROP_QUEUE(128, 3),
+    GFK_PROP_QUEUE(128, 4),
+    GFK_PROP_QUEUE(128, 5),
+    GFK_PROP_QUEUE(128, 6),
+    GFK_PROP_QUEUE(256, 2),
 };
 constexpr int kPropVariants = sizeof(kDunkinVariants) / sizeof(kDunkinVariants[0]);
 #undef GFK_PROP_SHAPE
@@ -380,102 +606,119 @@ bool prop_variant_shape(int variant, int* threads, int* blocks_per_sm, int* ilp,
     const PropVariant& v = kDunkinVariants[variant];
     *threads = v.threads;
     *blocks_per_sm = v.minb;
-    *ilp = v.ilp;
-    *sweeps = v.sweeps;
+    *ilp = 1;
+    *sweeps = v.threads / 16;  // a panel of 128 wavenumbers per 16 threads
     *persistent = v.persistent ? 1 : 0;
     return true;
 }
 
 void launch_prop(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, const cd* wc2, int nf,
-                 int max_nk, const cd* C, int formulation, cd* rem, int* status, int variant, const SliceOut* slice,
-                 unsigned int* queue) {
+                 int max_nk, const cd* C, int formulation, const double* tab, cd* rem, int* status, int variant,
+                 const SliceOut* slice, unsigned int* queue) {
     if (nf <= 0 || max_nk <= 0) return;
     const SliceOut so = slice ? *slice : SliceOut{};
     if (formulation == 0) {
         dim3 grid((max_nk + 127) / 128, nf);
         if (slice)
-            k_prop<0, 128, 1, 1, 1, true><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, rem, status, so, PropQueue{});
+            k_prop<0, 128, 1, true><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
         else
-            k_prop<0, 128, 1, 1, 1, false><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, rem, status, so, PropQueue{});
+            k_prop<0, 128, 1, false><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
         return;
     }
     if (variant < 0 || variant >= kPropVariants) variant = 0;
-    if (kDunkinVariants[variant].persistent && !queue) variant = 1;  // no queue: the same block shape, one item each
+    if (kDunkinVariants[variant].persistent && !queue) variant = 2;  // no queue: one item per block
     const PropVariant& v = kDunkinVariants[variant];
-    const int per_item = v.threads * v.ilp * v.sweeps;
+    const int per_item = v.threads * 8;
     const int runs = (max_nk + per_item - 1) / per_item;
     const PropFn fn = slice ? v.fn_slice : v.fn;
     if (v.persistent) {
         const PropQueue q{queue, nf * runs, runs};
-        fn<<<std::min(persistent_grid(variant, slice != nullptr), nf * runs), v.threads, 0, s>>>(lc, media, fd, wc2, C,
-                                                                                              rem, status, so, q);
+        fn<<<std::min(persistent_grid(variant, slice != nullptr), nf * runs), v.threads, 0, s>>>(
+            lc, media, fd, wc2, C, tab, rem, status, so, q);
     } else {
-        fn<<<dim3(runs, nf), v.threads, 0, s>>>(lc, media, fd, wc2, C, rem, status, so, PropQueue{});
+        fn<<<dim3(runs, nf), v.threads, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
     }
 }
 
 void launch_prop_rows(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, int nf,
-                      const cd* wc2, cd* C, int formulation, cd* ku, int* status, const RowItems& it) {
+                      const cd* wc2, cd* C, int formulation, const double* tab, cd* ku, int* status,
+                      const RowItems& it) {
     if (nf <= 0) return;
-    const dim3 grid(it.items + (nf + 127) / 128, it.kc / 128);
+    const int extra = (nf + 127) / 128;
+    const dim3 grid(it.items + extra, it.kc / 128);
     if (formulation == 0)
-        k_prop_rows<0><<<grid, 128, 0, s>>>(lc, media, fd, nf, wc2, C, ku, status, it);
+        k_prop_rows<0, false><<<grid, 128, 0, s>>>(lc, media, fd, nf, wc2, C, tab, ku, status, it);
+    else if (tab)
+        k_prop_rows<1, true><<<dim3(it.items + extra, (it.kc + 1023) / 1024), 128, 0, s>>>(lc, media, fd, nf, wc2, C,
+                                                                                        tab, ku, status, it);
     else
-        k_prop_rows<1><<<grid, 128, 0, s>>>(lc, media, fd, nf, wc2, C, ku, status, it);
+        k_prop_rows<1, false><<<grid, 128, 0, s>>>(lc, media, fd, nf, wc2, C, tab, ku, status, it);
 }
 
 // ------------------------------------------------- fused propagator + sum --
 //
 // For a handful of ranges the wavenumber sum is a dot product per range: each
-// thread accumulates its integrand values k u - C times the Hankel weights
-// W[k][0..nr) over kFuseSweeps wavenumbers, the block reduces over its
-// kFuseSweeps x 128 wavenumbers in a fixed order (warp tree, then warps), and
-// one partial per (row, k block, range) is written. The
-// integrand never reaches HBM; k_fused_finish adds the partials in block
+// thread accumulates its values k u - C times the Hankel weights over its
+// block's 1024 wavenumbers (8 panels), the block reduces in a fixed order (warp
+// tree, then warps), and one partial per (row, k block, range) is written. A
+// panel taken from its nodes is never interpolated: the weights of its 128
+// wavenumbers are carried over to the nodes once per grid (k_panel_weights).
+// The integrand never reaches HBM; k_fused_finish adds the partials in block
 // order (deterministic) and the closed k = 0 panel (fk.go:529-532).
 
 constexpr int kFuseThreads = 128;
-constexpr int kFuseSweeps = 8;  // a block covers kFuseSweeps x 128 wavenumbers of its row
+constexpr int kFuseSpan = 8 * kFuseThreads;  // wavenumbers of its row a block covers
+
+// Wp[panel][48][nr]: sum over the panel's wavenumbers of the interpolation
+// matrix times W, for the 16-node and then the 32-node fit.
+__global__ void k_panel_weights(const double* __restrict__ W, const double* __restrict__ tab, int nk, int nr,
+                                double* __restrict__ Wp) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int panels = (nk + kPanel - 1) / kPanel;
+    if (t >= (int64_t)panels * 48 * nr) return;
+    const int q = (int)(t % nr), j = (int)(t / nr % 48), p = (int)(t / nr / 48);
+    double s = 0.0;
+    for (int i = 0; i < kPanel && p * kPanel + i < nk; i++) {
+        const double m = j < kPanelE ? tab[kPtFragE + panel_frag(i, j, kPanelE)]
+                                     : tab[kPtFragN + panel_frag(i, j - kPanelE, kPanelN)];
+        s = fma(m, W[(size_t)(p * kPanel + i) * nr + q], s);
+    }
+    Wp[t] = s;
+}
+
+size_t panel_weight_count(int nk, int nr) { return (size_t)((nk + kPanel - 1) / kPanel) * 48 * nr; }
+
+void launch_panel_weights(cudaStream_t s, const double* W, const double* tab, int nk, int nr, double* Wp) {
+    const size_t n = panel_weight_count(nk, nr);
+    k_panel_weights<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(W, tab, nk, nr, Wp);
+}
 
 template <int NR>
 __global__ __launch_bounds__(kFuseThreads, 4) void k_prop_fused(const LayerC* __restrict__ lc,
                                                                 const MediumP* __restrict__ media,
                                                                 const FreqDesc* __restrict__ fd,
                                                                 const cd* __restrict__ wc2, const cd* __restrict__ C,
-                                                                const double* __restrict__ W, int nr, int nkb,
+                                                                const double* __restrict__ tab,
+                                                                const double* __restrict__ W,
+                                                                const double* __restrict__ Wp, int nr, int nkb,
                                                                 cd* __restrict__ partial, int* __restrict__ status) {
-    __shared__ LayerC s_lc[kMaxLayers];
+    __shared__ PropSmem<kFuseThreads, false> sm;
     __shared__ double s_red[2 * NR][kFuseThreads / 32];
     const int f = blockIdx.y;
     const FreqDesc fdesc = fd[f];
     const MediumP med = media[fdesc.soil];
     const int nl = med.count;
-    for (int l = threadIdx.x; l < nl; l += blockDim.x) s_lc[l] = lc[fdesc.lc_off + l];
+    for (int l = threadIdx.x; l < nl; l += blockDim.x) sm.lc[l] = lc[fdesc.lc_off + l];
     __syncthreads();
     const int n = fdesc.kfar > 0 ? fdesc.nk : 0;
-    const cd wc2f = wc2[f], cf = C[f];
     double acc[2 * NR];
 #pragma unroll
     for (int q = 0; q < 2 * NR; q++) acc[q] = 0.0;
-    // kFuseSweeps wavenumbers per thread, 128 apart, summed in order: one
-    // layer-table load and one block reduction per 512 wavenumbers
-#pragma unroll 1
-    for (int sweep = 0; sweep < kFuseSweeps; sweep++) {
-        const int i = (blockIdx.x * kFuseSweeps + sweep) * kFuseThreads + threadIdx.x + 1;
-        if (i > n) break;
-        const double k = (double)i * fdesc.dk;
-        cd r = k * dunkin_u(s_lc, nl, wc2f, k, med.mu_ref) - cf;
-        if (!finite_cd(r)) {
-            atomicOr(status + f, kStNonfinite);
-            r = mk(0.0);
-        }
-#pragma unroll
-        for (int j = 0; j < NR; j++) {
-            const double w = j < nr ? W[(size_t)(i - 1) * nr + j] : 0.0;
-            acc[2 * j] = fma(r.re, w, acc[2 * j]);
-            acc[2 * j + 1] = fma(r.im, w, acc[2 * j + 1]);
-        }
-    }
+    double mre = 0.0, mim = 0.0;
+    int bad = 0;
+    panel_item<kFuseThreads, NR, true>(tab, sm, nl, med.mu_ref, wc2[f], C[f], fdesc.dk, n, blockIdx.x * kFuseSpan, n,
+                                       nullptr, W, Wp, nr, acc, mre, mim, bad);
+    if (bad) atomicOr(status + f, bad);
     // warp tree, then the block's warps in order: a fixed summation order
 #pragma unroll
     for (int q = 0; q < 2 * NR; q++)
@@ -514,19 +757,19 @@ __global__ void k_fused_finish(const cd* __restrict__ partial, const cd* __restr
 int fused_max_ranges() { return 8; }
 
 void launch_prop_fused(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, const cd* wc2,
-                       int nf, int nk, const cd* C, const double* W, const double* ranges, int nr, cd* partial,
-                       int* status, cd* G) {
+                       int nf, int nk, const cd* C, const double* tab, const double* W, const double* Wp,
+                       const double* ranges, int nr, cd* partial, int* status, cd* G) {
     if (nf <= 0 || nk <= 0 || nr <= 0 || nr > 8) return;
-    const int nkb = (nk + kFuseThreads * kFuseSweeps - 1) / (kFuseThreads * kFuseSweeps);
+    const int nkb = (nk + kFuseSpan - 1) / kFuseSpan;
     dim3 grid(nkb, nf);
     if (nr <= 1)
-        k_prop_fused<1><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, W, nr, nkb, partial, status);
+        k_prop_fused<1><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, tab, W, Wp, nr, nkb, partial, status);
     else if (nr <= 2)
-        k_prop_fused<2><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, W, nr, nkb, partial, status);
+        k_prop_fused<2><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, tab, W, Wp, nr, nkb, partial, status);
     else if (nr <= 4)
-        k_prop_fused<4><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, W, nr, nkb, partial, status);
+        k_prop_fused<4><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, tab, W, Wp, nr, nkb, partial, status);
     else
-        k_prop_fused<8><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, W, nr, nkb, partial, status);
+        k_prop_fused<8><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, tab, W, Wp, nr, nkb, partial, status);
     const int64_t nt = (int64_t)nf * nr;
     k_fused_finish<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(partial, C, ranges, fd, nf, nr, nkb, G);
 }
@@ -583,14 +826,6 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 }  // namespace qd
-
-// Not volatile: the result is used, and the compiler may move the next
-// step's fragment loads ahead of these MMAs.
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-        : "+d"(c0), "+d"(c1)
-        : "d"(a), "d"(b));
-}
 
 template <int TNW>
 __global__ __launch_bounds__(qd::THREADS, TNW == 8 ? 1 : 2) void k_quad_gemm(const cd* __restrict__ rem,

@@ -42,7 +42,7 @@ struct RowItems {
 int rows_item_size(long long wavenumbers, int nr);
 
 // rem[fd[f].off + i - 1] = k_i u(k_i, f) - C_f for i = 1..nk, k_i = i dk.
-// `variant` picks one of prop_variant_count() launch shapes of the Dunkin
+// tab: the panel table (gfk_panel.cuh). `variant` picks one of prop_variant_count() launch shapes of the Dunkin
 // kernel; the persistent ones (prop_variant_persistent) take their items from
 // `queue`, one zeroed word (without one they run as one item per block).
 // With `slice` (a shared grid, rows fd[f].off = f nk) each row is also cut into
@@ -50,12 +50,12 @@ int rows_item_size(long long wavenumbers, int nr);
 // slice->rowmax and slice->done must be zero for the launch's rows (the
 // launch leaves done at zero again).
 void launch_prop(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, const cd* wc2, int nf,
-                 int max_nk, const cd* C, int formulation, cd* rem, int* status, int variant = 0,
+                 int max_nk, const cd* C, int formulation, const double* tab, cd* rem, int* status, int variant = 0,
                  const SliceOut* slice = nullptr, unsigned int* queue = nullptr);
 int prop_variant_count();
 bool prop_variant_persistent(int variant);
 // threads per block, blocks per SM it is compiled for, wavenumbers per thread
-// at a time, 128-wavenumber runs per item, persistent or one item per block
+// at a time, 128-wavenumber panels per item, persistent or one item per block
 bool prop_variant_shape(int variant, int* threads, int* blocks_per_sm, int* ilp, int* sweeps, int* persistent);
 
 // Tensor-core quadrature (gfk_quad_tc.cu): exact int8 slices of the integrand
@@ -79,11 +79,14 @@ int quad_tc_selftest_timeout(cudaStream_t s, long long wait_cycles, int* timed_o
 int quad_tc_splits(int M, int N, int Kp);  // split count filling the SMs for one chunk shape
 
 // Shared grid, nr <= fused_max_ranges(): propagator and wavenumber sum in one
-// pass (the integrand stays on chip); partial holds nf x ceil(nk/128) x nr.
+// pass (the integrand stays on chip); partial holds nf x ceil(nk/1024) x nr.
+// Wp: the weights carried over to the panels' nodes (launch_panel_weights).
 int fused_max_ranges();
+size_t panel_weight_count(int nk, int nr);
+void launch_panel_weights(cudaStream_t s, const double* W, const double* tab, int nk, int nr, double* Wp);
 void launch_prop_fused(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, const cd* wc2,
-                       int nf, int nk, const cd* C, const double* W, const double* ranges, int nr, cd* partial,
-                       int* status, cd* G);
+                       int nf, int nk, const cd* C, const double* tab, const double* W, const double* Wp,
+                       const double* ranges, int nr, cd* partial, int* status, cd* G);
 
 // W[(i-1) nr + j] = w_i J0(k_i r_j) dk, w = 1/2 at i = nk.
 void launch_j0_table(cudaStream_t s, const double* ranges, int nr, int nk, double dk, double* W);
@@ -101,9 +104,10 @@ void launch_quad_finish(cudaStream_t s, const cd* part, int splits, const cd* C,
 
 // Per-frequency grids: ku[fd[f].off + i - 1] = k_i u(k_i, f) over items, with
 // the static coefficients C; then the sum of ku - C with J0 evaluated in the
-// loop; part holds items x nr.
+// loop; part holds items x nr. Without tab every wavenumber is solved.
 void launch_prop_rows(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, int nf,
-                      const cd* wc2, cd* C, int formulation, cd* ku, int* status, const RowItems& it);
+                      const cd* wc2, cd* C, int formulation, const double* tab, cd* ku, int* status,
+                      const RowItems& it);
 void launch_quad_rows(cudaStream_t s, const cd* ku, const cd* C, const double* ranges, int nf, int nr,
                       const FreqDesc* fd, const RowItems& it, cd* part, cd* G);
 

@@ -201,7 +201,7 @@ extern "C" int gfk_vertical_displacement_multi_noalloc(const gfk_medium* m, cons
     int kc = gfk::rows_item_size(g.samples, nr);
     while ((size_t)((g.samples + kc - 1) / kc) > fit) kc *= 2;
     const gfk::RowItems it{nullptr, nullptr, 0, 0, (g.samples + kc - 1) / kc, kc};
-    gfk::launch_prop_rows(strm, d_lc, d_medium, d_row, 1, d_wc2, d_C, form, d_rem, d_status, it);
+    gfk::launch_prop_rows(strm, d_lc, d_medium, d_row, 1, d_wc2, d_C, form, nullptr, d_rem, d_status, it);
     gfk::launch_quad_rows(strm, d_rem, d_C, d_r, 1, nr, d_row, it, reinterpret_cast<cd*>(base + part_off), d_G);
     ok(cudaGetLastError());
     int flags = 0;

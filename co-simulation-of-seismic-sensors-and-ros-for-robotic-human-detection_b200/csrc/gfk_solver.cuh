@@ -336,33 +336,6 @@ GFK_HD cd dunkin_u(const LayerC* L, int n, cd wc2, double k, double mu_ref) {
     return cdiv_fast(m[3], (kTwoPi * mu_ref * k) * m[4]);
 }
 
-// Two wavenumbers of one frequency in lockstep through the layers: two
-// independent dependency chains per thread, for latency hiding at low occupancy.
-GFK_HD void dunkin_u2(const LayerC* L, int n, cd wc2, double k0, double k1, double mu_ref, cd& u0, cd& u1) {
-    const cd c20 = wc2 * rcp_(k0 * k0);
-    const cd c21 = wc2 * rcp_(k1 * k1);
-    const int top0 = start_layer(L, n, c20, k0), top1 = start_layer(L, n, c21, k1);
-    cd m0[5], m1[5];
-    {
-        Terms t0 = layer_terms(L[top0], c20);
-        Terms t1 = layer_terms(L[top1], c21);
-        decaying_minors(t0, m0);
-        decaying_minors(t1, m1);
-    }
-    for (int i = (top0 > top1 ? top0 : top1) - 1; i >= 0; i--) {
-        if (i < top0) {
-            Terms t0 = layer_terms(L[i], c20);
-            dunkin_layer_up(t0, k0 * L[i].h, m0, i % kRenormEvery == 0);
-        }
-        if (i < top1) {
-            Terms t1 = layer_terms(L[i], c21);
-            dunkin_layer_up(t1, k1 * L[i].h, m1, i % kRenormEvery == 0);
-        }
-    }
-    u0 = cdiv_fast(m0[3], (kTwoPi * mu_ref * k0) * m0[4]);
-    u1 = cdiv_fast(m1[3], (kTwoPi * mu_ref * k1) * m1[4]);
-}
-
 // ------------------------------------------------------ reference direct --
 
 struct M4 {

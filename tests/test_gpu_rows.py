@@ -4,7 +4,7 @@ test_gpu_parity."""
 import numpy as np
 import pytest
 
-from conftest import as_tuples, rel_l2
+from conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
 
