@@ -148,10 +148,11 @@ GFK_HD Terms layer_terms(const LayerC& L, cd c2) {
     t.ieb = crcp_(eb);
     if (cnorm1(eb) < 0.35) {
         const cd A = crcp_(1.0 + t.ra), B = crcp_(1.0 + t.rb);
-        t.u1 = kap * A + t.ra * B;
-        t.delta = eb * (B - kap * A);
+        const cd kA = kap * A;
+        t.u1 = cmadd(t.ra, B, kA);
+        t.delta = eb * (B - kA);
     } else {
-        t.u1 = (1.0 - t.ra * t.rb) * t.ieb;
+        t.u1 = cnmadd(t.ra, t.rb, mk(1.0)) * t.ieb;
         t.delta = (eb - ea) * crcp_(t.ra + t.rb);
     }
     t.x2 = 2.0 * t.u1 - 1.0;
@@ -218,14 +219,14 @@ GFK_HD void apply_step(const Step& s, cd m[5], bool renorm) {
     // adj(B03) = [[mu' rb, 0], [-mu'(1 + rb^2), 1]], adj(B12) = [[-mu' x2, u1], [-2 mu' ra, ra]]
     const cd v03 = mra * m[2];
     const cd v12 = mrb * m[3];
-    const cd T00 = u1 * m[1] - mx2 * m[0];
-    const cd T01 = ra * m[1] - mra2 * m[0];
-    const cd T10 = -(mx2 * m[1] + u1 * m[4]);
-    const cd T11 = -(mra2 * m[1] + ra * m[4]);
+    const cd T00 = cmul2_sub(u1, m[1], mx2, m[0]);
+    const cd T01 = cmul2_sub(ra, m[1], mra2, m[0]);
+    const cd nT10 = cmul2_add(mx2, m[1], u1, m[4]);
+    const cd nT11 = cmul2_add(mra2, m[1], ra, m[4]);
     const cd v01 = mrb * T00;
     const cd v02 = mrb * T01;
-    const cd v13 = mq * T00 - T10;
-    const cd v23 = mq * T01 - T11;
+    const cd v13 = cmadd(mq, T00, nT10);
+    const cd v23 = cmadd(mq, T01, nT11);
     // y = C(S)^T v (F-basis pairs)
     const cd sab = v02 - v13, pab = v02 + v13, scd = v03 - v12, pcd = v03 + v12;
     const cd y0 = sab + scd;
@@ -236,16 +237,15 @@ GFK_HD void apply_step(const Step& s, cd m[5], bool renorm) {
     const cd y5 = sab - scd;
     // middle minors Z = P Y Q^T, Y = [[y1, y2], [y3, y4]]; the outer pairs
     // scale by 1 and (Ea Eb)^2
-    const cd p00 = Eb * y1 - W * y3, p01 = Eb * y2 - W * y4;
+    const cd p00 = cmul2_sub(Eb, y1, W, y3), p01 = cmul2_sub(Eb, y2, W, y4);
     const cd p10 = Ea * y3, p11 = Ea * y4;
-    const cd z1 = Ea * p00 - W * p01;
+    const cd z1 = cmul2_sub(Ea, p00, W, p01);
     const cd z2 = Eb * p01;
-    const cd z3 = Ea * p10 - W * p11;
+    const cd z3 = cmul2_sub(Ea, p10, W, p11);
     const cd z4 = Eb * p11;
-    const cd z5 = s.EaEb2 * y5;
-    const cd z0 = y0;
     // w = C(S) z (G-basis pairs)
-    const cd s05 = z0 + z5, d05 = z0 - z5, s23 = z2 + z3, d23 = z2 - z3;
+    const cd s05 = cmadd(s.EaEb2, y5, y0), d05 = cnmadd(s.EaEb2, y5, y0);  // y0 +- z5
+    const cd s23 = z2 + z3, d23 = z2 - z3;
     const cd w01 = 2.0 * z1;
     const cd w02 = s05 + d23;
     const cd w03 = d05 - s23;
@@ -254,14 +254,14 @@ GFK_HD void apply_step(const Step& s, cd m[5], bool renorm) {
     const cd w23 = -2.0 * z4;
     // m = C(G) w: pure pairs by the block determinants, mixed
     // [[w01, w02], [-w13, -w23]] to B03 (.) B12^T (its (3,1) entry, -M13, not formed)
-    const cd U00 = ra * w01 - u1 * w02;
-    const cd U01 = mra2 * w01 - mx2 * w02;
-    const cd U11 = mx2 * w23 - mra2 * w13;
+    const cd U00 = cmul2_sub(ra, w01, u1, w02);
+    const cd U01 = cmul2_sub(mra2, w01, mx2, w02);
+    const cd U11 = cmul2_sub(mx2, w23, mra2, w13);
     m[0] = U00;
     m[1] = U01;
     m[2] = mrb * w03;
     m[3] = mra * w12;
-    m[4] = -(mq * U01 + mrb * U11);
+    m[4] = -cmul2_add(mq, U01, mrb, U11);
     // renormalise by a power of two (exact; the common scale cancels)
     if (!renorm) return;
     double mx = 0.0;
