@@ -142,7 +142,7 @@ void launch_static(cudaStream_t s, const LayerC* lc, const MediumP* media, const
 //
 // The work item is (row f, run): 8 panels of 128 wavenumbers per 128 threads
 // (gfk_panel.cuh). Pass 0 solves the 16 first nodes of every panel, one per
-// thread, a half-warp per panel, which tests its coefficients by shuffles;
+// thread, a half-warp per panel, which tests its coefficients;
 // pass 1 the other 16 nodes of the panels that may be served by 32; the passes
 // after that every wavenumber of the remaining panels. One loop holds the
 // three, so the solve is compiled once. The interpolation of the accepted
@@ -152,8 +152,8 @@ void launch_static(cudaStream_t s, const LayerC* lc, const MediumP* media, const
 // fragments come from L1).
 //
 // k_prop serves one item per block (blockIdx = (run, f)); k_prop_q is
-// persistent: each resident block takes items from a device queue in row order
-// until none are left. The row's layer constants are staged in shared memory.
+// persistent: each resident block takes items from a device queue, last row
+// first, until none are left. The row's layer constants are staged in shared memory.
 // Launch shapes are template parameters; the plan times them once and keeps
 // the fastest. The direct formulation solves every wavenumber: its parity with
 // the reference includes the digits its eigenbasis loses.
@@ -226,33 +226,36 @@ __device__ __forceinline__ double half_max(double v) {
 // end or n). NR = 0: the integrand goes to row[]; NR > 0: each value is added
 // to acc times the range's weights, W[wavenumber][nr] or, for a whole panel,
 // Wp[panel][48][nr] (the weights carried over to its 16 or 32 nodes). SUB: the
-// values are k u - c, else k u.
-template <int THREADS, int NR, bool SUB, class SMEM>
+// values are k u - c, else k u. WIDE: a warp per panel solves all 32 nodes in
+// the first pass (the same decisions from the same values): more solves, but
+// an item is half as many wavenumbers and passes, for banks of few items.
+template <int THREADS, bool WIDE, int NR, bool SUB, class SMEM>
 __device__ __forceinline__ void panel_item(const double* __restrict__ tab, SMEM& sm, int nl, double mu_ref, cd w2,
                                            cd c, double d, int n, int base, int lim, cd* __restrict__ row,
                                            const double* __restrict__ W, const double* __restrict__ Wp, int nr,
                                            double* acc, double& mre, double& mim, int& bad) {
-    constexpr int PANELS = THREADS / 16;
-    const int tid = threadIdx.x, hp = tid >> 4, hj = tid & 15;
+    constexpr int PANELS = THREADS / (WIDE ? 32 : 16);
+    const int tid = threadIdx.x, hp = tid >> (WIDE ? 5 : 4), hj = tid & 15;
     const int pa = base + kPanel * hp;
     const bool use = pa < lim && n - pa >= kPanelLeast;
     const double cabs1 = SUB ? cnorm1(c) : 0.0;
-    cd first = mk(0.0);
+    cd first = mk(0.0), other = mk(0.0);
     double big = 0.0;
     bool more = false;
     int mode = 0;
-    unsigned direct = 0;
+    unsigned direct = 0;  // panels to be solved, or (64 threads) their halves
 #pragma unroll 1
     for (int pass = 0;; pass++) {
         double x;  // wavenumber / d
         bool live;
         int i = 0;
         if (pass < 2) {
-            live = pass == 0 ? use : more;
-            x = fma(64.0, tab[kPtX + pass * kPanelE + hj], (double)pa + 64.5);
+            live = pass == 0 ? use : !WIDE && more;
+            x = fma(64.0, tab[kPtX + (WIDE ? tid & 31 : pass * kPanelE + hj)], (double)pa + 64.5);
         } else {
             if (direct == 0) break;
-            i = base + kPanel * (__ffs(direct) - 1) + (tid & (kPanel - 1)) + 1;
+            constexpr int STEP = THREADS < kPanel ? THREADS : kPanel;
+            i = base + STEP * (__ffs(direct) - 1) + (tid & (STEP - 1)) + 1;
             if constexpr (THREADS > kPanel) {  // the upper threads take the next panel
                 const unsigned rest = direct & (direct - 1);
                 if (tid >= kPanel) i = rest ? base + kPanel * (__ffs(rest) - 1) + (tid & (kPanel - 1)) + 1 : n + 1;
@@ -269,6 +272,12 @@ __device__ __forceinline__ void panel_item(const double* __restrict__ tab, SMEM&
             if (SUB) r -= c;
         }
         if (pass == 0) {
+            if constexpr (NR == 0) sm.nodes[hp * kNodeStride + (WIDE ? tid & 31 : hj)] = r;
+            if (WIDE) {  // both half-warps hold the panel's pairs of first and other nodes from here on
+                const cd v = r;
+                r = cd{__shfl_sync(0xffffffffu, v.re, hj), __shfl_sync(0xffffffffu, v.im, hj)};
+                other = cd{__shfl_sync(0xffffffffu, v.re, 16 + hj), __shfl_sync(0xffffffffu, v.im, 16 + hj)};
+            }
             first = r;
             big = half_max(cnorm1(r));
             const cd v[1] = {r};
@@ -280,8 +289,8 @@ __device__ __forceinline__ void panel_item(const double* __restrict__ tab, SMEM&
             const float s = (float)(1.0 / scale), tl = (float)tail * s, q = tl / ((float)mid * s);
             const float room = (float)(10.0 * kPanelTol) / tl, q2 = q * q, q4 = q2 * q2;
             more = use && !mode && q < 1.0f && q4 * q4 <= room * room * room;
-            if (NR == 0) sm.nodes[hp * kNodeStride + hj] = r;
         } else if (pass == 1) {
+            if (WIDE) r = other;
             if (__any_sync(0xffffffffu, more)) {
                 const double m2 = half_max(cnorm1(r));
                 const cd v[2] = {first, r};
@@ -305,13 +314,14 @@ __device__ __forceinline__ void panel_item(const double* __restrict__ tab, SMEM&
                         }
                 }
             } else {
-                sm.nodes[hp * kNodeStride + kPanelE + hj] = r;
+                if (!WIDE) sm.nodes[hp * kNodeStride + kPanelE + hj] = r;
             }
             if (hj == 0) sm.mode[hp] = (unsigned char)mode;
             __syncthreads();
 #pragma unroll
             for (int p = 0; p < PANELS; p++)
-                if (sm.mode[p] == 0 && base + kPanel * p < lim) direct |= 1u << p;
+                if (sm.mode[p] == 0 && base + kPanel * p < lim)
+                    direct |= THREADS >= kPanel ? 1u << p : (base + kPanel * p + 64 < lim ? 3u : 1u) << (2 * p);
         } else if (live) {
             if (!(isfinite(r.re) && isfinite(r.im))) { bad |= kStNonfinite; r = mk(0.0); }
             if constexpr (NR > 0) {
@@ -329,11 +339,12 @@ __device__ __forceinline__ void panel_item(const double* __restrict__ tab, SMEM&
         }
     }
     if constexpr (NR == 0) {
-        // warp w holds points 32 w' .. + 31 (w' = w mod 4) of 4 panels at a time:
-        // C fragment row = point, columns 2 (panel) + part
-        const int lane = tid & 31, wq = (tid >> 5) & 3;
+        // a warp takes points 32 wq .. + 31 of 4 panels at a time: C fragment
+        // row = point, columns 2 (panel) + part
+        const int lane = tid & 31;
 #pragma unroll 1
-        for (int g = (tid >> 7) * 4; g < PANELS; g += THREADS / kPanel * 4) {
+        for (int job = tid >> 5; job < PANELS; job += THREADS / 32) {
+            const int g = job & ~3, wq = job & 3;
             const int bm = sm.mode[g + (lane >> 3)];
             const bool any1 = __any_sync(0xffffffffu, bm == 1), any2 = __any_sync(0xffffffffu, bm == 2);
             if (!any1 && !any2) continue;
@@ -376,7 +387,7 @@ __device__ __forceinline__ void panel_item(const double* __restrict__ tab, SMEM&
 }
 
 // `stage`: the block's staged layer constants are not row f's (uniform).
-template <int FORM, int THREADS, bool SLICE>
+template <int FORM, int THREADS, bool WIDE, bool SLICE>
 __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const MediumP* __restrict__ media,
                                           const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2,
                                           const cd* __restrict__ C, const double* __restrict__ tab,
@@ -410,8 +421,8 @@ __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const M
             mim = fabs(r.im);
         }
     } else {
-        panel_item<THREADS, 0, true>(tab, sm, nl, mu_ref, wc2[f], c, d, n, run * THREADS * 8, n, row, nullptr, nullptr,
-                                     0, nullptr, mre, mim, bad);
+        panel_item<THREADS, WIDE, 0, true>(tab, sm, nl, mu_ref, wc2[f], c, d, n, run * THREADS * (WIDE ? 4 : 8), n, row,
+                                           nullptr, nullptr, 0, nullptr, mre, mim, bad);
     }
     if (bad) atomicOr(status + f, bad);
     if constexpr (SLICE) {
@@ -454,7 +465,7 @@ __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const M
     }
 }
 
-template <int FORM, int THREADS, int MINB, bool SLICE>
+template <int FORM, int THREADS, int MINB, bool WIDE, bool SLICE>
 __global__ __launch_bounds__(THREADS, MINB) void k_prop(const LayerC* __restrict__ lc,
                                                        const MediumP* __restrict__ media,
                                                        const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2,
@@ -462,8 +473,8 @@ __global__ __launch_bounds__(THREADS, MINB) void k_prop(const LayerC* __restrict
                                                        cd* __restrict__ rem, int* __restrict__ status, SliceOut so,
                                                        PropQueue) {
     __shared__ PropSmem<THREADS, SLICE> sm;
-    prop_item<FORM, THREADS, SLICE>(lc, media, fd, wc2, C, tab, rem, status, so, blockIdx.y, blockIdx.x, gridDim.x,
-                                    true, sm);
+    prop_item<FORM, THREADS, WIDE, SLICE>(lc, media, fd, wc2, C, tab, rem, status, so, gridDim.y - 1 - blockIdx.y, blockIdx.x,
+                                    gridDim.x, true, sm);
 }
 
 // Rows of uneven length: block (item, y) serves the y-th run of 128
@@ -503,7 +514,7 @@ __global__ __launch_bounds__(128, FORM == 0 ? 1 : 5) void k_prop_rows(const Laye
     int bad = 0;
     if constexpr (PANEL) {
         double mre = 0.0, mim = 0.0;
-        panel_item<128, 0, false>(tab, sm, med.count, med.mu_ref, wc2[f], mk(0.0), fdesc.dk, fdesc.nk, base, lim, row,
+        panel_item<128, false, 0, false>(tab, sm, med.count, med.mu_ref, wc2[f], mk(0.0), fdesc.dk, fdesc.nk, base, lim, row,
                                   nullptr, nullptr, 0, nullptr, mre, mim, bad);
     } else {
         const int i = base + threadIdx.x + 1;
@@ -525,10 +536,10 @@ __global__ __launch_bounds__(128, FORM == 0 ? 1 : 5) void k_prop_rows(const Laye
     if (bad) atomicOr(status + f, bad);
 }
 
-// Persistent: items (f, run) in row order from q.next (zero at launch), so a
+// Persistent: items (f, run), row by row, from q.next (zero at launch), so a
 // row's items run together and the row is sliced while it is in L2. Blocks
 // never wait for one another; each leaves when the queue is empty.
-template <int FORM, int THREADS, int MINB, bool SLICE>
+template <int FORM, int THREADS, int MINB, bool WIDE, bool SLICE>
 __global__ __launch_bounds__(THREADS, MINB) void k_prop_q(const LayerC* __restrict__ lc,
                                                          const MediumP* __restrict__ media,
                                                          const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2,
@@ -543,8 +554,10 @@ __global__ __launch_bounds__(THREADS, MINB) void k_prop_q(const LayerC* __restri
         __syncthreads();
         const int item = sm.item;
         if (item >= q.items) return;
-        const int f = item / q.runs, run = item - f * q.runs;
-        prop_item<FORM, THREADS, SLICE>(lc, media, fd, wc2, C, tab, rem, status, so, f, run, q.runs, f != cur, sm);
+        // the last rows first: a medium's higher frequencies, whose poles reach
+        // further, are its costlier rows, and the queue ends on cheap items
+        const int rf = item / q.runs, run = item - rf * q.runs, f = q.items / q.runs - 1 - rf;
+        prop_item<FORM, THREADS, WIDE, SLICE>(lc, media, fd, wc2, C, tab, rem, status, so, f, run, q.runs, f != cur, sm);
         cur = f;
     }
 }
@@ -555,21 +568,29 @@ using PropFn = void (*)(const LayerC*, const MediumP*, const FreqDesc*, const cd
 struct PropVariant {
     PropFn fn, fn_slice;  // without and with the fused slicing
     int threads, minb;
+    bool wide;        // all 32 nodes in the first pass
     bool persistent;  // k_prop_q: one block per resident slot, items from a queue
 };
-#define GFK_PROP_SHAPE(T, B) {k_prop<1, T, B, false>, k_prop<1, T, B, true>, T, B, false}
-#define GFK_PROP_QUEUE(T, B) {k_prop_q<1, T, B, false>, k_prop_q<1, T, B, true>, T, B, true}
+#define GFK_PROP_SHAPE(T, B, W) {k_prop<1, T, B, W, false>, k_prop<1, T, B, W, true>, T, B, W, false}
+#define GFK_PROP_QUEUE(T, B, W) {k_prop_q<1, T, B, W, false>, k_prop_q<1, T, B, W, true>, T, B, W, true}
+// 80 registers spill up to 220 bytes a thread and still lead: six blocks of four
+// warps hide the FP64 latency. On the 2048-row graded bank (ms, with the sum's
+// 0.48): 256 threads at 3 blocks per SM 2.44, 128 at 4, 5, 6, 7 blocks 2.50,
+// 2.45, 2.41, 2.46, 64 at 10 and 12 2.51, 2.52; one item per warp without
+// barriers 2.82 (an item is then up to 20 solves in series). All nodes at once:
+// a 301-row bank of three items a row 0.134 -> 0.113 ms.
 const PropVariant kDunkinVariants[] = {
-    GFK_PROP_SHAPE(128, 3),  // <= 168 registers, 12 warps/SM
-    GFK_PROP_SHAPE(128, 4),  // <= 128 registers
-    GFK_PROP_SHAPE(128, 5),  // <= 96 registers
-    GFK_PROP_SHAPE(128, 6),  // <= 80 registers
-    GFK_PROP_SHAPE(256, 2),  // 16 panels per item
-    GFK_PROP_QUEUE(128, 3),
-    GFK_PROP_QUEUE(128, 4),
-    GFK_PROP_QUEUE(128, 5),
-    GFK_PROP_QUEUE(128, 6),
-    GFK_PROP_QUEUE(256, 2),
+    GFK_PROP_SHAPE(64, 12, false),  // 4 panels per item, <= 80 registers
+    GFK_PROP_SHAPE(128, 5, false),  // 8 panels per item, <= 96 registers
+    GFK_PROP_SHAPE(128, 6, false),  // <= 80 registers
+    GFK_PROP_SHAPE(256, 3, false),  // 16 panels per item
+    GFK_PROP_SHAPE(128, 5, true),   // 4 panels per item, all nodes at once
+    GFK_PROP_SHAPE(256, 2, true),
+    GFK_PROP_QUEUE(64, 12, false),
+    GFK_PROP_QUEUE(128, 5, false),
+    GFK_PROP_QUEUE(128, 6, false),
+    GFK_PROP_QUEUE(256, 3, false),
+    GFK_PROP_QUEUE(128, 5, true),
 };
 constexpr int kPropVariants = sizeof(kDunkinVariants) / sizeof(kDunkinVariants[0]);
 #undef GFK_PROP_SHAPE
@@ -607,7 +628,7 @@ bool prop_variant_shape(int variant, int* threads, int* blocks_per_sm, int* ilp,
     *threads = v.threads;
     *blocks_per_sm = v.minb;
     *ilp = 1;
-    *sweeps = v.threads / 16;  // a panel of 128 wavenumbers per 16 threads
+    *sweeps = v.threads / (v.wide ? 32 : 16);  // a panel of 128 wavenumbers per 16 threads
     *persistent = v.persistent ? 1 : 0;
     return true;
 }
@@ -620,15 +641,15 @@ void launch_prop(cudaStream_t s, const LayerC* lc, const MediumP* media, const F
     if (formulation == 0) {
         dim3 grid((max_nk + 127) / 128, nf);
         if (slice)
-            k_prop<0, 128, 1, true><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
+            k_prop<0, 128, 1, false, true><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
         else
-            k_prop<0, 128, 1, false><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
+            k_prop<0, 128, 1, false, false><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
         return;
     }
     if (variant < 0 || variant >= kPropVariants) variant = 0;
     if (kDunkinVariants[variant].persistent && !queue) variant = 2;  // no queue: one item per block
     const PropVariant& v = kDunkinVariants[variant];
-    const int per_item = v.threads * 8;
+    const int per_item = v.threads * (v.wide ? 4 : 8);
     const int runs = (max_nk + per_item - 1) / per_item;
     const PropFn fn = slice ? v.fn_slice : v.fn;
     if (v.persistent) {
@@ -694,7 +715,7 @@ void launch_panel_weights(cudaStream_t s, const double* W, const double* tab, in
 }
 
 template <int NR>
-__global__ __launch_bounds__(kFuseThreads, 4) void k_prop_fused(const LayerC* __restrict__ lc,
+__global__ __launch_bounds__(kFuseThreads, NR <= 2 ? 6 : 4) void k_prop_fused(const LayerC* __restrict__ lc,
                                                                 const MediumP* __restrict__ media,
                                                                 const FreqDesc* __restrict__ fd,
                                                                 const cd* __restrict__ wc2, const cd* __restrict__ C,
@@ -704,7 +725,7 @@ __global__ __launch_bounds__(kFuseThreads, 4) void k_prop_fused(const LayerC* __
                                                                 cd* __restrict__ partial, int* __restrict__ status) {
     __shared__ PropSmem<kFuseThreads, false> sm;
     __shared__ double s_red[2 * NR][kFuseThreads / 32];
-    const int f = blockIdx.y;
+    const int f = gridDim.y - 1 - blockIdx.y;  // the costlier rows first
     const FreqDesc fdesc = fd[f];
     const MediumP med = media[fdesc.soil];
     const int nl = med.count;
@@ -716,7 +737,7 @@ __global__ __launch_bounds__(kFuseThreads, 4) void k_prop_fused(const LayerC* __
     for (int q = 0; q < 2 * NR; q++) acc[q] = 0.0;
     double mre = 0.0, mim = 0.0;
     int bad = 0;
-    panel_item<kFuseThreads, NR, true>(tab, sm, nl, med.mu_ref, wc2[f], C[f], fdesc.dk, n, blockIdx.x * kFuseSpan, n,
+    panel_item<kFuseThreads, false, NR, true>(tab, sm, nl, med.mu_ref, wc2[f], C[f], fdesc.dk, n, blockIdx.x * kFuseSpan, n,
                                        nullptr, W, Wp, nr, acc, mre, mim, bad);
     if (bad) atomicOr(status + f, bad);
     // warp tree, then the block's warps in order: a fixed summation order
