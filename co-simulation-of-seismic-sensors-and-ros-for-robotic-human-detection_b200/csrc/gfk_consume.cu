@@ -15,9 +15,9 @@
 //              inverse-transformed (1/n), the first `length` samples kept.
 //
 // One thread per bin builds the tables (the unwrap is sequential in range);
-// one block per query range builds its half spectrum in shared memory and runs
-// the inverse real transform there as an n/2-point complex FFT (gfk_fft.cuh),
-// n = the bank's Samples <= 4096.
+// one block per query range forms its half spectrum in registers and runs the
+// inverse real transform as an n/2-point complex FFT (gfk_fft.cuh), n = the
+// bank's Samples <= 4096.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -76,72 +76,92 @@ struct ImpulseArgs {
     double* out;            // [nq][length]
 };
 
+// The tables' values of bin k at a query's two ranges.
+struct Bracketed {
+    double l0, l1, p0, p1;
+};
+
+// H_k of one query: the response between its two ranges, times i w and the
+// sensor's response, tapered.
+__device__ __forceinline__ cd half_spectrum(const ImpulseArgs& a, const Bracketed& t, double frac, int k) {
+    if (k == 0 || t.l0 == kNegInf || t.l1 == kNegInf) return mk(0.0);
+    const double pi = 3.14159265358979323846;
+    const double lm = t.l0 + frac * (t.l1 - t.l0), ph = t.p0 + frac * (t.p1 - t.p0);
+    double sn, cs;
+    sincos(ph, &sn, &cs);
+    const double f = k * a.fs / a.n, nyq = a.fs / 2, taper_from = 0.8 * nyq;
+    double mg = exp(lm);
+    if (f > taper_from) mg *= 0.5 * (1.0 + cos(pi * (f - taper_from) / (nyq - taper_from)));
+    cd h = mk(mg * cs, mg * sn);
+    if (a.velocity) h = cmul_i((2.0 * pi * f) * h);
+    if (a.sensor) h = h * a.sensor[k];
+    return h;
+}
+
 // The inverse real transform of the half spectrum H_0..H_m (m = n/2) as one
 // complex transform of size m (the even/odd split of the output): with
 // w = e^{2 pi i / n},
 //   Z_k = (H_k + conj(H_{m-k})) + i w^k (H_k - conj(H_{m-k})),  k < m,
 //   z = IDFT_m(Z) / n  gives  y_2j = Re z_j,  y_2j+1 = Im z_j,
-// and IDFT_m(Z) = conj(DFT_m(conj Z)). Shared memory: m + 1 values.
-__global__ void __launch_bounds__(kThreads) k_impulse(ImpulseArgs a) {
-    extern __shared__ cd x[];  // [m + 1]: H, then conj(Z) (bit-reversed), then its transform
+// and IDFT_m(Z) = conj(DFT_m(conj Z)). A thread forms H_k and H_{m-k} and stores
+// the pair's conj(Z); the last pass writes the samples. Bound by the FP64 work
+// of the spectrum (an exponential and a sine-cosine per bin) beside 65 KB of
+// table reads (L2) per query of 2049 bins; 8192 queries of 1024 samples took
+// 803 us with the spectrum staged through shared memory and a radix-2
+// transform (11 passes), 285 us now; 32 warps an SM (64 registers) beat 24 by 3%.
+__global__ void __launch_bounds__(kThreads, 4) k_impulse(ImpulseArgs a) {
+    extern __shared__ cd x[];  // fft_room(m): conj(Z), then the passes
     const int q = blockIdx.x;
     const int n = a.n, m = n / 2;
     const int logm = 31 - __clz(m);
     const int lo = a.lo[q];
-    const int hi = a.count == 1 ? lo : lo + 1;
+    const size_t row0 = (size_t)lo * a.bins, row1 = a.count == 1 ? row0 : row0 + a.bins;
     const double frac = a.frac[q];
-    const double nyq = a.fs / 2, taper_from = 0.8 * nyq;
-    const double pi = 3.14159265358979323846;
-    for (int k = threadIdx.x; k <= m; k += blockDim.x) {
-        cd h = mk(0.0);
-        const double f = k * a.fs / n;
-        if (k > 0 && k < a.bins) {
-            const size_t i0 = (size_t)lo * a.bins + k, i1 = (size_t)hi * a.bins + k;
-            if (a.logmag[i0] != kNegInf && a.logmag[i1] != kNegInf) {
-                const double lm = a.logmag[i0] + frac * (a.logmag[i1] - a.logmag[i0]);
-                const double ph = a.phase[i0] + frac * (a.phase[i1] - a.phase[i0]);
-                double sn, cs;
-                sincos(ph, &sn, &cs);
-                const double mg = exp(lm);
-                h = mk(mg * cs, mg * sn);
-                if (a.velocity) h = mk(0.0, 2.0 * pi * f) * h;
-                if (a.sensor) h = h * a.sensor[k];
-            }
-            if (f > taper_from) h = h * (0.5 * (1.0 + cos(pi * (f - taper_from) / (nyq - taper_from))));
-        }
-        if (k == 0 || k == m) h.im = 0.0;  // the real transform reads only their real parts
-        x[k] = h;
-    }
-    __syncthreads();
-    // conj(Z_k) and conj(Z_{m-k}) by the thread that owns the pair (k, m - k)
+    auto fetch = [&](int k) {  // bins = m + 1: every k of [0, m] is in the tables
+        return Bracketed{a.logmag[row0 + k], a.logmag[row1 + k], a.phase[row0 + k], a.phase[row1 + k]};
+    };
+    // the next pair's table values are in flight while a pair is formed
+    Bracketed t1 = fetch(min((int)threadIdx.x, m)), t2 = fetch(max(m - (int)threadIdx.x, 0));
     for (int k = threadIdx.x; k <= m / 2; k += blockDim.x) {
         const int k2 = m - k;
-        const cd hk = x[k], hk2 = x[k2];
+        const Bracketed c1 = t1, c2 = t2;
+        const int kn = k + blockDim.x;
+        if (kn <= m / 2) {
+            t1 = fetch(kn);
+            t2 = fetch(m - kn);
+        }
+        cd hk = half_spectrum(a, c1, frac, k), hk2 = half_spectrum(a, c2, frac, k2);
+        if (k == 0) hk.im = hk2.im = 0.0;  // the real transform reads only their real parts
         const cd wk = mk(a.tw[k].re, -a.tw[k].im);  // e^{2 pi i k / n}
         const cd zk = (hk + mk(hk2.re, -hk2.im)) + cmul_i(wk * (hk - mk(hk2.re, -hk2.im)));
-        x[k] = mk(zk.re, -zk.im);
-        if (k > 0 && k < m / 2) {
-            const cd wk2 = mk(a.tw[k2].re, -a.tw[k2].im);
+        x[fft_at(k)] = mk(zk.re, -zk.im);
+        if (k > 0 && k < k2) {
+            const cd wk2 = mk(-wk.re, wk.im);  // e^{2 pi i (m - k) / n} = -conj(w^k)
             const cd zk2 = (hk2 + mk(hk.re, -hk.im)) + cmul_i(wk2 * (hk2 - mk(hk.re, -hk.im)));
-            x[k2] = mk(zk2.re, -zk2.im);
+            x[fft_at(k2)] = mk(zk2.re, -zk2.im);
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; logm > 0 && i < m; i += blockDim.x) {  // into bit-reversed order
-        const int r = bitrev(i, logm);
-        if (i < r) {
-            const cd t = x[i];
-            x[i] = x[r];
-            x[r] = t;
-        }
-    }
-    __syncthreads();
-    fft_pow2_dit_inplace(x, m, a.tw, n);
     const double inv = 1.0 / n;
-    for (int t = threadIdx.x; t < a.length; t += blockDim.x) {
-        const cd w = x[t >> 1];
-        a.out[(size_t)q * a.length + t] = ((t & 1) ? -w.im : w.re) * inv;
-    }
+    double* const out = a.out + (size_t)q * a.length;
+    const bool pairs = (a.length & 1) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
+    fft_block(x, logm, a.tw, n, [&](int i, cd v) {
+        const int t = 2 * i;
+        if (t >= a.length) return;
+        if (pairs) {
+            *reinterpret_cast<double2*>(out + t) = make_double2(v.re * inv, -v.im * inv);
+        } else {
+            out[t] = v.re * inv;
+            if (t + 1 < a.length) out[t + 1] = -v.im * inv;
+        }
+    });
+}
+
+void launch_impulse(cudaStream_t s, const ImpulseArgs& a, int nq) {
+    const int m = a.n / 2;
+    const int smem = fft_room(m) * (int)sizeof(cd);  // at most 36.9 KB: no opt-in
+    static_assert(fft_room(kMaxSamples / 2) * sizeof(cd) <= 48 * 1024, "shared memory");
+    k_impulse<<<nq, m >= 256 ? m / 8 : 32, smem, s>>>(a);
 }
 
 }  // namespace consume
@@ -284,15 +304,11 @@ int gfk_bank_impulse_responses(gfk_ctx* ctx, const float* payload, int32_t count
         CS_CUDA(ctx, cudaMallocAsync(&d_sensor.p, (size_t)bins * 2 * sizeof(double), s));
         CS_CUDA(ctx, cudaMemcpyAsync(d_sensor.p, sensor, (size_t)bins * 2 * sizeof(double), cudaMemcpyHostToDevice, s));
     }
-    const size_t smem = (size_t)(samples / 2 + 1) * sizeof(cd);
-    if (smem > 48 * 1024)
-        CS_CUDA(ctx, cudaFuncSetAttribute(gfk::consume::k_impulse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
     gfk::consume::ImpulseArgs a{t.logmag, t.phase, count, bins, samples, length,
                                 static_cast<const int*>(d_lo.p), static_cast<const double*>(d_frac.p),
                                 static_cast<const cd*>(d_sensor.p), velocity, fs_hz,
                                 static_cast<const cd*>(d_tw.p), static_cast<double*>(d_out.p)};
-    gfk::consume::k_impulse<<<nq, gfk::consume::kThreads, smem, s>>>(a);
+    gfk::consume::launch_impulse(s, a, nq);
     ctx->launches++;
     CS_CUDA(ctx, cudaGetLastError());
     CS_CUDA(ctx, cudaMemcpyAsync(out, d_out.p, (size_t)nq * length * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -428,13 +444,9 @@ int gfk_bank_device_impulse_responses(gfk_bank_dev* b, const double* ranges, int
         if (int st = grow(ctx, &b->d_out, &b->out_cap, (size_t)nq * length)) return st;
         dst = b->d_out;
     }
-    const size_t smem = (size_t)(b->samples / 2 + 1) * sizeof(cd);
-    if (smem > 48 * 1024)
-        CS_CUDA(ctx, cudaFuncSetAttribute(gfk::consume::k_impulse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
     gfk::consume::ImpulseArgs a{b->t.logmag, b->t.phase, b->count, b->bins, b->samples, length, b->d_lo, b->d_frac,
                                 d_sensor, velocity, b->fs, reinterpret_cast<const cd*>(b->d_tw), dst};
-    gfk::consume::k_impulse<<<nq, gfk::consume::kThreads, smem, s>>>(a);
+    gfk::consume::launch_impulse(s, a, nq);
     ctx->launches++;
     CS_CUDA(ctx, cudaGetLastError());
     if (!out_on_device)

@@ -35,30 +35,116 @@ __device__ inline cd* fft_pow2(cd* x, cd* y, int n, const cd* __restrict__ tw) {
     return src;
 }
 
-// In-place iterative radix-2 decimation in time (Cooley-Tukey): x holds the
-// input in bit-reversed order (element k at index bitrev(k)); the forward
-// transform (e^{-i}) ends in x in natural order. Half the shared memory of
-// fft_pow2; every thread of the block must call it.
-__device__ inline void fft_pow2_dit_inplace(cd* x, int n, const cd* __restrict__ tw, int tw_n = 0) {
-    // tw holds e^{-2 pi i m / tw_n}, m < tw_n / 2 (tw_n = n by default; a
-    // multiple of n reuses a larger transform's table)
-    const int tn = tw_n > 0 ? tw_n : n;
-    for (int len = 2; len <= n; len <<= 1) {
-        const int half = len >> 1, step = tn / len;
-        for (int j = threadIdx.x; j < n / 2; j += blockDim.x) {
-            const int pos = j & (half - 1);
-            const int i0 = ((j - pos) << 1) + pos;
-            const cd w = tw[pos * step];
-            const cd a = x[i0];
-            const cd b = x[i0 + half] * w;
-            x[i0] = a + b;
-            x[i0 + half] = a - b;
+// Forward DFT (e^{-i}) of R = 2, 4 or 8 values in registers.
+template <int R>
+__device__ __forceinline__ void dft_small(cd (&v)[R]) {
+    if constexpr (R == 2) {
+        const cd t = v[1];
+        v[1] = v[0] - t;
+        v[0] = v[0] + t;
+    } else if constexpr (R == 4) {
+        const cd a = v[0] + v[2], b = v[0] - v[2], c = v[1] + v[3], d = v[1] - v[3];
+        v[0] = a + c;
+        v[2] = a - c;
+        v[1] = cd{b.re + d.im, b.im - d.re};  // b - i d
+        v[3] = cd{b.re - d.im, b.im + d.re};
+    } else {
+        static_assert(R == 8, "radix");
+        cd e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        dft_small<4>(e);
+        dft_small<4>(o);
+        constexpr double h = 0.70710678118654752440;
+        o[1] = cd{h * (o[1].re + o[1].im), h * (o[1].im - o[1].re)};
+        o[2] = cd{o[2].im, -o[2].re};
+        o[3] = cd{h * (o[3].im - o[3].re), -h * (o[3].re + o[3].im)};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            v[i] = e[i] + o[i];
+            v[i + 4] = e[i] - o[i];
         }
-        __syncthreads();
     }
 }
 
-// Index of element k in the bit-reversed order of a 2^logn record.
-__device__ __forceinline__ int bitrev(int k, int logn) { return (int)(__brev((unsigned)k) >> (32 - logn)); }
+// Element i of a record in shared memory lies at fft_at(i): a gap of one
+// (16-byte) element after every eight, so that neither the radix-8 passes'
+// strided stores nor their contiguous loads conflict.
+__device__ __forceinline__ int fft_at(int i) { return i + (i >> 3); }
+__host__ __device__ constexpr int fft_room(int m) { return m + m / 8 + 1; }
+
+// One radix-R Stockham pass over m values by max(32, m / 8) threads, each with
+// up to 8 / R butterflies: loads x, then (all threads) emit(element, value)
+// for every output. tw[q] = e^{-2 pi i q / tn}, q < tn/2, tn a multiple of m;
+// ns is the product of the radices before. Twiddles: w, w^2, w^4 from the
+// table, the others as their products.
+template <int R, class Emit>
+__device__ __forceinline__ void fft_pass(const cd* x, int m, int ns, const cd* __restrict__ tw, int tn, Emit emit) {
+    constexpr int B = 8 / R;
+    const int stride = m / R, tid = threadIdx.x, nt = m >= 256 ? m / 8 : 32;
+    cd v[B][R];
+#pragma unroll
+    for (int b = 0; b < B; b++) {
+        const int j = tid + b * nt;
+        if (j < stride) {
+#pragma unroll
+            for (int r = 0; r < R; r++) v[b][r] = x[fft_at(j + r * stride)];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < B; b++) {
+        const int j = tid + b * nt;
+        if (j >= stride) continue;
+        const int k = j & (ns - 1);
+        if (ns > 1) {
+            const int q = k * (tn / (ns * R));
+            cd w[R];
+            w[1] = tw[q];
+            if constexpr (R >= 4) {
+                w[2] = tw[2 * q];  // 2 q < 2 tn / R <= tn / 2
+                w[3] = w[1] * w[2];
+            }
+            if constexpr (R == 8) {
+                const int q4 = 4 * q;  // < tn / 2
+                w[4] = tw[q4];
+                w[5] = w[4] * w[1];
+                w[6] = w[4] * w[2];
+                w[7] = w[4] * w[3];
+            }
+#pragma unroll
+            for (int r = 1; r < R; r++) v[b][r] = v[b][r] * w[r];
+        }
+        dft_small<R>(v[b]);
+        const int d = (j - k) * R + k;
+#pragma unroll
+        for (int r = 0; r < R; r++) emit(d + r * ns, v[b][r]);
+    }
+}
+
+// Forward transform (e^{-i}) of the m = 2^logm values at x[fft_at(i)], the last
+// pass handing its outputs, in natural order, to emit(i, value) instead of
+// shared memory. The block has max(32, m / 8) threads; all must call it, with
+// x written and a barrier passed. Every pass but the first is radix 8: a third of the
+// passes (and of the shared-memory traffic and barriers) of radix 2.
+template <class Emit>
+__device__ __forceinline__ void fft_block(cd* x, int logm, const cd* __restrict__ tw, int tn, Emit emit) {
+    const int m = 1 << logm;
+    const int head = logm % 3;
+    auto keep = [&](int i, cd v) { x[fft_at(i)] = v; };
+    if (logm == 0) {
+        if (threadIdx.x == 0) emit(0, x[0]);
+        return;
+    }
+    if (logm == 1) return fft_pass<2>(x, m, 1, tw, tn, emit);
+    if (logm == 2) return fft_pass<4>(x, m, 1, tw, tn, emit);
+    int ns = 1;
+    if (head == 1) fft_pass<2>(x, m, 1, tw, tn, keep), ns = 2;
+    if (head == 2) fft_pass<4>(x, m, 1, tw, tn, keep), ns = 4;
+    if (head) __syncthreads();
+    for (; ns * 8 < m; ns *= 8) {
+        fft_pass<8>(x, m, ns, tw, tn, keep);
+        __syncthreads();
+    }
+    fft_pass<8>(x, m, ns, tw, tn, emit);
+}
 
 }  // namespace gfk
