@@ -214,7 +214,9 @@ struct gfk_plan {
     int kc = 0;
     std::vector<int> item_row, row_begin;
     int *d_item_row = nullptr, *d_row_begin = nullptr;
-    // device
+    // device: the tables and small buffers lie in one allocation, the large
+    // buffers in one each (Layout)
+    std::vector<void*> owned;
     gfk::LayerP* d_lp = nullptr;
     gfk::MediumP* d_media = nullptr;
     gfk::FreqDesc* d_fd = nullptr;
@@ -248,6 +250,8 @@ struct gfk_plan {
     // CUDA graph of one whole execute
     bool use_graph = false;
     cudaGraphExec_t gexec = nullptr;
+    // built, executed and freed by one call: no timing events
+    bool transient = false;
     // timing
     std::vector<TimedSeg> segs;
     size_t seg_next = 0;
@@ -266,18 +270,74 @@ void plan_free(gfk_plan* p) {
     cudaStream_t s = p->ctx ? p->ctx->stream : nullptr;
     if (p->gexec) cudaGraphExecDestroy(p->gexec);
     if (p->ev_chunk) cudaEventDestroy(p->ev_chunk);
-    void* ptrs[] = {p->d_lp, p->d_media,  p->d_fd, p->d_ranges, p->d_lc,     p->d_wc2,    p->d_C,
-                    p->d_rem, p->d_G,     p->d_status, p->d_A, p->d_rowexp, p->d_rowmax, p->d_partial,
-                    p->d_ksum, p->d_queue, p->d_item_row, p->d_row_begin};
-    for (void* q : ptrs)
-        if (q) cudaFreeAsync(q, s);
+    for (void* q : p->owned) cudaFreeAsync(q, s);
     p->wts.reset();  // the weights go with their last plan (or stay in the context's cache)
     for (auto& sg : p->segs) {
         cudaEventDestroy(sg.a);
         cudaEventDestroy(sg.b);
     }
-    if (s) cudaStreamSynchronize(s);
+    // a transient plan's call has waited for its download
+    if (s && !(p->transient && p->executed)) cudaStreamSynchronize(s);
 }
+
+// The device buffers of a plan, requested one by one and made together: what
+// fits 1 MB shares one allocation, and its uploads, first in it, one copy (up
+// to 256 KB of them, staged on the host). A small bank's 17 buffers and 4
+// uploads cost its call more than the kernels.
+struct Layout {
+    struct Item {
+        void** ptr;
+        size_t bytes;
+        const void* src;
+    };
+    static constexpr size_t kSmall = size_t(1) << 20, kStaged = size_t(256) << 10;
+    std::vector<Item> items;
+    template <class T>
+    void add(T** ptr, size_t count, const T* src = nullptr) {
+        items.push_back({reinterpret_cast<void**>(ptr), std::max<size_t>(count, 1) * sizeof(T), count ? src : nullptr});
+    }
+    static size_t room(size_t bytes) { return (bytes + 255) & ~size_t(255); }
+
+    int make(gfk_ctx* ctx, std::vector<void*>& owned) {
+        auto grab = [&](void** ptr, size_t bytes) -> int {
+            cudaError_t e = cudaMallocAsync(ptr, bytes, ctx->stream);
+            if (e != cudaSuccess) {
+                *ptr = nullptr;
+                return fail(ctx, GFK_ENOMEM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+            }
+            owned.push_back(*ptr);
+            return GFK_OK;
+        };
+        size_t up = 0, all = 0;
+        for (const Item& i : items)
+            if (i.src && i.bytes <= kSmall) up += room(i.bytes);
+        const bool staged = up <= kStaged;
+        for (const Item& i : items)
+            if (i.bytes <= kSmall) all += room(i.bytes);
+        unsigned char* base = nullptr;
+        if (all)
+            if (int st = grab(reinterpret_cast<void**>(&base), all)) return st;
+        std::vector<unsigned char> host(staged ? up : 0);
+        size_t at_up = 0, at = up;
+        for (const Item& i : items) {
+            if (i.bytes > kSmall) {
+                if (int st = grab(i.ptr, i.bytes)) return st;
+            } else {
+                size_t& pos = i.src ? at_up : at;
+                *i.ptr = base + pos;
+                if (i.src && staged) std::memcpy(host.data() + pos, i.src, i.bytes);
+                pos += room(i.bytes);
+            }
+            if (i.src && !(staged && i.bytes <= kSmall) &&
+                cudaMemcpyAsync(*i.ptr, i.src, i.bytes, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
+                return fail(ctx, GFK_ECUDA, "plan upload failed");
+        }
+        // pageable copies return with their source staged: `host` may go
+        if (staged && up && cudaMemcpyAsync(base, host.data(), up, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
+            return fail(ctx, GFK_ECUDA, "plan upload failed");
+        return GFK_OK;
+    }
+};
 
 template <class T>
 int dalloc(gfk_ctx* ctx, T** ptr, size_t count) {
@@ -323,6 +383,7 @@ int h2d(gfk_ctx* ctx, T* dst, const T* src, size_t count) {
 
 int begin_seg(gfk_plan* p, int kind, size_t* slot) {
     gfk_ctx* ctx = p->ctx;
+    if (p->transient) return GFK_OK;
     if (p->segs.size() < 256) {
         TimedSeg sg{kind, nullptr, nullptr, false};
         GFK_CUDA(ctx, cudaEventCreate(&sg.a));
@@ -347,6 +408,7 @@ int begin_seg(gfk_plan* p, int kind, size_t* slot) {
 }
 
 int end_seg(gfk_plan* p, size_t slot) {
+    if (p->transient) return GFK_OK;
     GFK_CUDA(p->ctx, cudaEventRecord(p->segs[slot].b, p->ctx->stream));
     p->segs[slot].pending = true;
     return GFK_OK;
@@ -586,29 +648,30 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
     // device buffers
     int st = GFK_OK;
     const size_t nfa = std::max(p->nf, 1);
-    if (!st) st = dalloc(ctx, &p->d_lp, std::max<size_t>(p->lp.size(), 1));
-    if (!st) st = dalloc(ctx, &p->d_media, (size_t)nsoil);
-    if (!st) st = dalloc(ctx, &p->d_fd, nfa);
-    if (!st) st = dalloc(ctx, &p->d_ranges, nr);
-    if (!st) st = dalloc(ctx, &p->d_lc, (size_t)std::max<int64_t>(lc_total, 1));
-    if (!st) st = dalloc(ctx, &p->d_wc2, nfa);
-    if (!st) st = dalloc(ctx, &p->d_C, nfa);
-    if (!st) st = dalloc(ctx, &p->d_G, nfa * nr);
-    if (!st) st = dalloc(ctx, &p->d_status, nfa);
-    if (!st) st = dalloc(ctx, &p->d_queue, 1);
+    Layout lay;
+    lay.add(&p->d_lp, p->lp.size(), p->lp.data());
+    lay.add(&p->d_media, (size_t)nsoil, p->media.data());
+    lay.add(&p->d_fd, (size_t)p->nf, p->fd.data());
+    lay.add(&p->d_ranges, (size_t)nr, p->ranges.data());
+    lay.add(&p->d_status, nfa);  // next to G: a small bank comes back in one copy
+    lay.add(&p->d_G, nfa * nr);
+    lay.add(&p->d_lc, (size_t)std::max<int64_t>(lc_total, 1));
+    lay.add(&p->d_wc2, nfa);
+    lay.add(&p->d_C, nfa);
+    lay.add(&p->d_queue, 1);
     if (p->fused) {
         int max_cnf = 0;
         for (size_t c = 0; c + 1 < p->chunk_begin.size(); c++)
             max_cnf = std::max(max_cnf, p->chunk_begin[c + 1] - p->chunk_begin[c]);
         const int nkb = (g_n + 1023) / 1024;
-        if (!st) st = dalloc(ctx, &p->d_partial, (size_t)max_cnf * nkb * nr);
-    } else if (!st) {
-        st = dalloc(ctx, &p->d_rem, (size_t)std::max<int64_t>(cap, 1));
+        lay.add(&p->d_partial, (size_t)max_cnf * nkb * nr);
+    } else {
+        lay.add(&p->d_rem, (size_t)std::max<int64_t>(cap, 1));
     }
     if (!p->shared) {
-        if (!st) st = dalloc(ctx, &p->d_item_row, p->item_row.size());
-        if (!st) st = dalloc(ctx, &p->d_row_begin, p->row_begin.size());
-        if (!st) st = dalloc(ctx, &p->d_ksum, (size_t)max_items * nr);
+        lay.add(&p->d_item_row, p->item_row.size(), p->item_row.data());
+        lay.add(&p->d_row_begin, p->row_begin.size(), p->row_begin.data());
+        lay.add(&p->d_ksum, (size_t)max_items * nr);
     }
     if (!st && p->shared && !p->tc) {
         const size_t count = (size_t)g_n * nr + (p->fused ? gfk::panel_weight_count(g_n, nr) : 0);
@@ -627,11 +690,11 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         // the propagator writes every digit of a chunk's rows up to Kp; rows
         // past a chunk's 2 cnf are computed by the sum but never stored, so
         // the planes need no clearing
-        st = dalloc(ctx, &p->d_A, (size_t)4 * p->Mp * p->Kp);
+        lay.add(&p->d_A, (size_t)4 * p->Mp * p->Kp);
         if (!st && !(st = plan_weights(p, gfk_weights::kDigits, g_n, g_kmax / g_n, (size_t)4 * p->Np * p->Kp)))
             p->d_B = static_cast<int8_t*>(p->wts->d);
-        if (!st) st = dalloc(ctx, &p->d_rowexp, (size_t)p->Mp);
-        if (!st) st = dalloc(ctx, &p->d_rowmax, (size_t)3 * max_cnf);  // row maxima, then finished-block counts
+        lay.add(&p->d_rowexp, (size_t)p->Mp);
+        lay.add(&p->d_rowmax, (size_t)3 * max_cnf);  // row maxima, then finished-block counts
     }
     if (!st && p->shared && !p->fused) {
         int max_cnf = 0;
@@ -641,16 +704,9 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         const int64_t per_split = (int64_t)max_cnf * nr;
         while (ks > 1 && ks * per_split * (int64_t)sizeof(cd) > (int64_t(512) << 20)) ks--;
         p->ksplit = ks;
-        if (ks > 1) st = dalloc(ctx, &p->d_ksum, (size_t)(ks * per_split));
+        if (ks > 1) lay.add(&p->d_ksum, (size_t)(ks * per_split));
     }
-    if (!st) st = h2d(ctx, p->d_lp, p->lp.data(), p->lp.size());
-    if (!st) st = h2d(ctx, p->d_media, p->media.data(), p->media.size());
-    if (!st) st = h2d(ctx, p->d_fd, p->fd.data(), p->fd.size());
-    if (!st) st = h2d(ctx, p->d_ranges, p->ranges.data(), nr);
-    if (!st && !p->shared) st = h2d(ctx, p->d_item_row, p->item_row.data(), p->item_row.size());
-    if (!st && !p->shared) st = h2d(ctx, p->d_row_begin, p->row_begin.data(), p->row_begin.size());
-    if (!st && cudaStreamSynchronize(ctx->stream) != cudaSuccess)  // host tables may be freed by the caller
-        st = fail(ctx, GFK_ECUDA, "plan upload failed");
+    if (!st) st = lay.make(ctx, p->owned);
     if (st) {
         plan_free(p);
         delete p;
@@ -938,10 +994,26 @@ int plan_download(gfk_plan* p, double* out, int32_t* status) {
     const int nf = p->nf, nr = p->nr;
     if (nf == 0) return GFK_OK;
     std::vector<int> dst(nf);
-    if (out)
-        GFK_CUDA(ctx, cudaMemcpyAsync(out, p->d_G, sizeof(cd) * (size_t)nf * nr, cudaMemcpyDeviceToHost, ctx->stream));
-    GFK_CUDA(ctx, cudaMemcpyAsync(dst.data(), p->d_status, sizeof(int) * nf, cudaMemcpyDeviceToHost, ctx->stream));
-    GFK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    // A small bank and its statuses, neighbours on the device, come back in one
+    // copy through the context's page-locked buffer (a pageable copy of 512 KB
+    // waits for its own staging).
+    const size_t gbytes = sizeof(cd) * (size_t)nf * nr, head = Layout::room(sizeof(int) * (size_t)nf);
+    const bool near = reinterpret_cast<unsigned char*>(p->d_G) == reinterpret_cast<unsigned char*>(p->d_status) + head;
+    if (out && near && head + gbytes <= gfk_ctx::kBounce && !ctx->bounce &&
+        cudaHostAlloc(&ctx->bounce, gfk_ctx::kBounce, cudaHostAllocDefault) != cudaSuccess) {
+        ctx->bounce = nullptr;
+        cudaGetLastError();
+    }
+    if (out && near && head + gbytes <= gfk_ctx::kBounce && ctx->bounce) {
+        GFK_CUDA(ctx, cudaMemcpyAsync(ctx->bounce, p->d_status, head + gbytes, cudaMemcpyDeviceToHost, ctx->stream));
+        GFK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        std::memcpy(dst.data(), ctx->bounce, sizeof(int) * (size_t)nf);
+        std::memcpy(out, static_cast<unsigned char*>(ctx->bounce) + head, gbytes);
+    } else {
+        if (out) GFK_CUDA(ctx, cudaMemcpyAsync(out, p->d_G, gbytes, cudaMemcpyDeviceToHost, ctx->stream));
+        GFK_CUDA(ctx, cudaMemcpyAsync(dst.data(), p->d_status, sizeof(int) * nf, cudaMemcpyDeviceToHost, ctx->stream));
+        GFK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    }
     int first = GFK_OK;
     std::string msg = ctx->last_error;
     for (int f = 0; f < nf; f++) {
@@ -1040,6 +1112,7 @@ int gfk_close(gfk_ctx* ctx) {
     ctx->plans.clear();
     ctx->weights.reset();
     if (ctx->panels) cudaFreeAsync(ctx->panels, ctx->stream);
+    if (ctx->bounce) cudaFreeHost(ctx->bounce);
     gfk_release_surrogates(ctx);
     gfk_release_banks(ctx);
     if (ctx->copy_stream) {
@@ -1261,6 +1334,7 @@ int gfk_bank_spectra(gfk_ctx* ctx, const gfk_medium* m, const gfk_solve* s, cons
     gfk_plan* p = nullptr;
     int st = plan_one(ctx, m, s, ranges, nr, freqs, nf, opt, kGridMulti, &p, overlap ? (nf + 1) / 2 : 0);
     if (st) return st;
+    p->transient = true;
     st = exec_download_overlapped(p, out, status_per_f);
     std::string msg = ctx->last_error;
     plan_free(p);
@@ -1280,6 +1354,7 @@ int gfk_bank_payload(gfk_ctx* ctx, const gfk_medium* m, const gfk_solve* s, cons
     gfk_plan* p = nullptr;
     int st = plan_one(ctx, m, s, ranges, nr, freqs, nf, opt, kGridMulti, &p);
     if (st) return st;
+    p->transient = true;
     st = plan_exec(p);
     std::vector<int32_t> stv(std::max(p->nf, 1), GFK_OK);
     int first = GFK_OK;
@@ -1337,6 +1412,7 @@ int gfk_vertical_displacement(gfk_ctx* ctx, const gfk_medium* m, const gfk_solve
     gfk_plan* p = nullptr;
     int st = plan_one(ctx, m, s, &range_m, 1, &freq_hz, 1, opt, kGridSingle, &p);
     if (st) return st;
+    p->transient = true;
     st = plan_exec(p);
     int32_t fst = 0;
     if (!st) st = plan_download(p, out, &fst);

@@ -198,7 +198,7 @@ class Medium:
             st = N.lib().gfk_vertical_displacement_multi(eng.ctx, ctypes.byref(cm), ctypes.byref(self._solve()),
                                                          _dp(r), len(r), float(freq), opt.c(), _dp(out))
         eng.check(st)
-        return out[0::2] + 1j * out[1::2]
+        return out.view(np.complex128)
 
     def bank_spectra(self, ranges, freqs, opt=None, raise_on_error=True, out=None):
         """VerticalDisplacementMulti at many frequencies in one GPU call, as
@@ -210,7 +210,8 @@ class Medium:
         opt = opt or Integration()
         r = np.ascontiguousarray(ranges, dtype=np.float64)
         f = np.ascontiguousarray(freqs, dtype=np.float64)
-        if out is None:
+        own = out is None
+        if own:
             out = np.zeros((len(f), 2 * len(r)))
         elif out.shape != (len(f), 2 * len(r)) or out.dtype != np.float64 or not out.flags.c_contiguous:
             raise ValueError("out must be a C-contiguous float64 array of shape (len(freqs), 2 len(ranges))")
@@ -222,7 +223,8 @@ class Medium:
                                           status.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)))
         if st and raise_on_error:
             eng.check(st)
-        return out[:, 0::2] + 1j * out[:, 1::2], status
+        spectra = out.view(np.complex128)  # the (re, im) pairs the ABI wrote
+        return spectra if own else spectra.copy(), status
 
     # -- helpers -----------------------------------------------------------
     def bank_payload(self, ranges, freqs, first_bin, bins, opt=None, raise_on_error=True, out=None):
