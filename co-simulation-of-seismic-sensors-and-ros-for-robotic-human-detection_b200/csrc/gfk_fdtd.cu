@@ -10,11 +10,15 @@
 //   stresses and memory variables fdtd.go:218-320
 //   surface velocity read-out     fdtd.go:330-345, Run's loop run.go:78-127
 //
-// Every phase of a step is a pure function of the previous phase's fields,
-// so each is one kernel over the grid (thread per cell, rows of the grid
-// contiguous): the velocity kernel also writes the prescribed surface
-// traction for this step, and the stress kernel also records the receivers
-// (their velocities are final by then). The arithmetic of every cell is the
+// Every phase of a step is a pure function of the previous phase's fields. A
+// step's new stresses depend on the old ones at most one cell away, so a block
+// that loads a tile and a halo of S cells can take S steps in shared memory
+// before it writes its tile back (k_tiles): one launch and one pass over memory
+// per S steps. The fields are double-buffered, because neighbouring tiles read
+// what this one writes. Where the second copy does not fit the device, each
+// phase is one kernel over the grid in place (k_velocities, which also writes
+// the prescribed surface traction, and k_stresses, which also records the
+// receivers: their velocities are final by then). The arithmetic of every cell is the
 // reference's, in the same order, except that divisions by the spacing, the
 // radius and the density are multiplications by precomputed reciprocals (the
 // same values to a rounding); FP64 throughout. Every 256 steps a max-speed
@@ -22,6 +26,7 @@
 #include <cmath>
 #include <complex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <math_constants.h>
@@ -174,6 +179,273 @@ __global__ void k_stresses(Args s, double dTdt, int step) {
         else
             s.trz[k] += s.dt * e;
     }
+}
+
+// ---- S steps per pass over memory --
+//
+// A block of 512 threads holds a 32 x 32 window of the fields: its tile of
+// (32 - 2S)^2 cells and the halo. A thread keeps its two cells' velocities,
+// stresses, memory variables and constants in registers; what the neighbours
+// read (velocities and stresses) and the C-PML variables also lie in shared
+// memory. Per step the valid part of the window shrinks by one cell on every
+// side that is not a domain edge; each phase runs over what is still valid.
+// Cells of the window's rim lack a neighbour and are skipped, which is what the
+// shrinking accounts for. With every field in shared memory a step read and
+// wrote it 50 times a cell and its bandwidth bound the step. On a
+// 281 x 201 grid one launch per phase left 14.9 us a step, nearly all launch
+// and L2 latency on 382 cells an SM; on 6 million cells the two phases moved
+// 208 bytes a cell and step, here 220 per 4 steps.
+
+constexpr int kTileW = 32, kTileCells = kTileW * kTileW, kTileThreads = kTileCells / 2, kOwn = 2;
+constexpr int kFields = 18, kMaxTileSteps = 10;
+enum : int { kVr, kVz, kTrr, kTqq, kTzz, kTrz, kRrr, kRqq, kRzz, kRrz, kTrrR, kTrzZ, kTrzR, kTzzZ, kVrR, kVzZ, kVzR, kVrZ };
+constexpr int kTileSmem = (6 + 8) * kTileCells * (int)sizeof(double);
+
+struct Tiles {
+    const double* in[kFields];
+    double* out[kFields];
+    const double* force;  // [steps + 1]
+    int S, n, step0;      // halo, steps of this launch (<= S), first step
+};
+
+template <bool LOSSY>
+__global__ void __launch_bounds__(kTileThreads, 1) k_tiles(Args s, Tiles t) {
+    extern __shared__ double sm[];
+    double* const vr = sm;
+    double* const vz = vr + kTileCells;
+    double* const trr = vz + kTileCells;
+    double* const tqq = trr + kTileCells;
+    double* const tzz = tqq + kTileCells;
+    double* const trz = tzz + kTileCells;
+    double* const psi = trz + kTileCells;  // [8]: kTrrR .. kVrZ
+    const int li = threadIdx.x & (kTileW - 1);
+    const int tw = kTileW - 2 * t.S;
+    const int x0 = blockIdx.x * tw, z0 = blockIdx.y * tw;  // the tile's first cell
+    const int gx = x0 - t.S, gz = z0 - t.S;                // the window's
+    const int i = gx + li, ic = min(max(i, 0), s.nr - 1);
+    // whether the window reaches the damped columns or rows (the psi fields are zero elsewhere)
+    const bool damp_r = gx + kTileW > min(s.fRi, s.fRh), damp_z = gz + kTileW > min(s.fZi, s.fZh);
+    const bool radial_psi[8] = {true, false, true, false, true, false, true, false};
+    // this thread's two cells (rows lj and lj + 16 of the window)
+    double ovr[kOwn], ovz[kOwn], orr[kOwn], oqq[kOwn], ozz[kOwn], orz[kOwn], m[kOwn][4];
+    double dt_rho[kOwn], dt_rhoZ[kOwn], lam[kOwn], mu[kOwn], muZ[kOwn];
+    double ps[kOwn][8];
+    // every load first, then the stores to shared memory: nothing tells the
+    // compiler that these pointers cannot reach shared memory, and it keeps the
+    // order of what might overlap (8 us a launch when they alternated)
+#pragma unroll
+    for (int c = 0; c < kOwn; c++) {
+        const int j = gz + (int)(threadIdx.x >> 5) + 16 * c;
+        const bool in = i >= 0 && i < s.nr && j >= 0 && j < s.nz;
+        const size_t k = (size_t)j * s.nr + i;
+        ovr[c] = in ? __ldg(t.in[kVr] + k) : 0.0;
+        ovz[c] = in ? __ldg(t.in[kVz] + k) : 0.0;
+        orr[c] = in ? __ldg(t.in[kTrr] + k) : 0.0;
+        oqq[c] = in ? __ldg(t.in[kTqq] + k) : 0.0;
+        ozz[c] = in ? __ldg(t.in[kTzz] + k) : 0.0;
+        orz[c] = in ? __ldg(t.in[kTrz] + k) : 0.0;
+#pragma unroll
+        for (int f = 0; f < 4; f++) m[c][f] = LOSSY && in ? __ldg(t.in[kRrr + f] + k) : 0.0;
+#pragma unroll
+        for (int f = 0; f < 8; f++) ps[c][f] = in && (radial_psi[f] ? damp_r : damp_z) ? __ldg(t.in[kTrrR + f] + k) : 0.0;
+        const int jc = min(max(j, 0), s.nz - 1);
+        dt_rho[c] = __ldg(s.dt_rho + jc);
+        dt_rhoZ[c] = __ldg(s.dt_rhoZ + jc);
+        lam[c] = __ldg(s.lamU + jc);
+        mu[c] = __ldg(s.muU + jc);
+        muZ[c] = __ldg(s.muZ + jc);
+    }
+#pragma unroll
+    for (int c = 0; c < kOwn; c++) {
+        const int e = ((threadIdx.x >> 5) + 16 * c) * kTileW + li;
+        vr[e] = ovr[c];
+        vz[e] = ovz[c];
+        trr[e] = orr[c];
+        tqq[e] = oqq[c];
+        tzz[e] = ozz[c];
+        trz[e] = orz[c];
+#pragma unroll
+        for (int f = 0; f < 8; f++)
+            if (radial_psi[f] ? damp_r : damp_z) psi[f * kTileCells + e] = ps[c][f];
+    }
+    const double ir_half = s.ir_half[ic], ir_int = s.ir_int[ic];
+    __syncthreads();
+    const bool source = gx <= 0 && gz <= 0;  // the window holds cell (0, 0)
+    auto damp = [&](int f, int e, const double* a, const double* b, int at, double d) {
+        return cpml(psi + (f - kTrrR) * kTileCells + e, a[at], b[at], d);
+    };
+    for (int n = 0; n < t.n; n++) {
+        const int step = t.step0 + n;
+        double traction = 0.0, rate = 0.0;  // at cell (0, 0) only
+        if (source) {
+            traction = -t.force[step] / s.src_area;
+            rate = (t.force[step + 1] - t.force[step]) / s.dt;
+        }
+        // the part still valid, in window coordinates
+        const int l0 = gx <= 0 ? -gx : n, l1 = gx + kTileW >= s.nr ? s.nr - gx : kTileW - n;
+        const int h0 = gz <= 0 ? -gz : n, h1 = gz + kTileW >= s.nz ? s.nz - gz : kTileW - n;
+        const bool col = li >= l0 && li < l1;
+        // both cells' neighbours are read before either is written (as above);
+        // an index past the window's rim is clamped, its cell is skipped below
+        double n1[kOwn], n2[kOwn], n3[kOwn], n4[kOwn], n5[kOwn];
+#pragma unroll
+        for (int c = 0; c < kOwn; c++) {
+            const int lj = (threadIdx.x >> 5) + 16 * c, e = lj * kTileW + li;
+            const int er = min(e + 1, kTileCells - 1), eu = max(e - kTileW, 0), ed = min(e + kTileW, kTileCells - 1);
+            n1[c] = trr[er];
+            n2[c] = tqq[er];
+            n3[c] = trz[eu];
+            n4[c] = tzz[ed];
+            n5[c] = trz[max(e - 1, 0)];
+        }
+#pragma unroll
+        for (int c = 0; c < kOwn; c++) {
+            const int lj = (threadIdx.x >> 5) + 16 * c, e = lj * kTileW + li, j = gz + lj;
+            if (!col || lj < h0 || lj >= h1 || i >= s.nr - 1 || j >= s.nz - 1) continue;
+            if (li + 1 < kTileW && (lj > 0 || j == 0)) {  // radial velocity
+                double dtrr = (n1[c] - orr[c]) * s.idr;
+                if (i >= s.fRh) dtrr += damp(kTrrR, e, s.aRh, s.bRh, i, dtrr);
+                double dtrz = j == 0 ? 2 * orz[c] * s.idz : (orz[c] - n3[c]) * s.idz;
+                if (j >= s.fZi) dtrz += damp(kTrzZ, e, s.aZi, s.bZi, j, dtrz);
+                const double hoop = 0.5 * ((orr[c] - oqq[c]) + (n1[c] - n2[c])) * ir_half;
+                ovr[c] += dt_rho[c] * (dtrr + dtrz + hoop);
+            }
+            if (lj + 1 < kTileW && (li > 0 || i == 0)) {  // vertical velocity
+                if (i == 0 && j == 0) ozz[c] = traction;  // fdtd.go:144
+                double dtzz = (n4[c] - ozz[c]) * s.idz;
+                if (j >= s.fZh) dtzz += damp(kTzzZ, e, s.aZh, s.bZh, j, dtzz);
+                double radial;
+                if (i == 0) {
+                    radial = 4 * orz[c] * s.idr;
+                } else {
+                    double d = (orz[c] - n5[c]) * s.idr;
+                    if (i >= s.fRi) d += damp(kTrzR, e, s.aRi, s.bRi, i, d);
+                    radial = d + 0.5 * (orz[c] + n5[c]) * ir_int;
+                }
+                ovz[c] += dt_rhoZ[c] * (dtzz + radial);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < kOwn; c++) {
+            const int e = ((threadIdx.x >> 5) + 16 * c) * kTileW + li;
+            vr[e] = ovr[c];
+            vz[e] = ovz[c];
+        }
+        __syncthreads();
+        // receivers of this tile's surface cells
+        if (z0 == 0)
+            for (int q = threadIdx.x; q < s.nrcv; q += kTileThreads) {
+                const int ri = s.cols[q];
+                if (ri < x0 || ri >= x0 + tw) continue;
+                const int e = -gz * kTileW + ri - gx;
+                double dvr, vrr;
+                if (ri == 0) {
+                    dvr = 2 * vr[e] / s.dr;
+                    vrr = dvr;
+                } else {
+                    dvr = (vr[e] - vr[e - 1]) / s.dr;
+                    vrr = 0.5 * (vr[e] + vr[e - 1]) / (double(ri) * s.dr);
+                }
+                const double l = s.lamU[0], g = s.muU[0];
+                const double dvz = -l / (l + 2 * g) * (dvr + vrr);
+                s.traces[(size_t)q * s.steps + step] = vz[e] - 0.5 * s.dz * dvz;
+            }
+#pragma unroll
+        for (int c = 0; c < kOwn; c++) {
+            const int lj = (threadIdx.x >> 5) + 16 * c, e = lj * kTileW + li;
+            n1[c] = vr[max(e - 1, 0)];
+            n2[c] = vz[max(e - kTileW, 0)];
+            n3[c] = vz[min(e + 1, kTileCells - 1)];
+            n4[c] = vr[min(e + kTileW, kTileCells - 1)];
+        }
+#pragma unroll
+        for (int c = 0; c < kOwn; c++) {
+            const int lj = (threadIdx.x >> 5) + 16 * c, e = lj * kTileW + li, j = gz + lj;
+            if (!col || lj < h0 || lj >= h1) continue;
+            const double lam2mu = lam[c] + 2 * mu[c];
+            if ((li > 0 || i == 0) && (lj > 0 || j == 0)) {  // normal stresses
+                double dvr, vrr;
+                if (i == 0) {
+                    dvr = 2 * ovr[c] * s.idr;
+                    vrr = dvr;
+                } else {
+                    dvr = (ovr[c] - n1[c]) * s.idr;
+                    vrr = 0.5 * (ovr[c] + n1[c]) * ir_int;
+                }
+                if (i >= s.fRi) dvr += damp(kVrR, e, s.aRi, s.bRi, i, dvr);
+                double dvz;
+                if (j == 0) {
+                    const double applied = i == 0 ? rate : 0.0;
+                    dvz = (applied - lam[c] * (dvr + vrr)) / lam2mu;
+                } else {
+                    dvz = (ovz[c] - n2[c]) * s.idz;
+                    if (j >= s.fZi) dvz += damp(kVzZ, e, s.aZi, s.bZi, j, dvz);
+                }
+                const double err = lam2mu * dvr + lam[c] * (vrr + dvz);
+                const double eqq = lam[c] * (dvr + dvz) + lam2mu * vrr;
+                orr[c] += s.dt * (LOSSY ? err + relax(s, &m[c][0], err) : err);
+                oqq[c] += s.dt * (LOSSY ? eqq + relax(s, &m[c][1], eqq) : eqq);
+                if (j != 0) {
+                    const double ezz = lam[c] * (dvr + vrr) + lam2mu * dvz;
+                    ozz[c] += s.dt * (LOSSY ? ezz + relax(s, &m[c][2], ezz) : ezz);
+                }
+            }
+            if (i < s.nr - 1 && j < s.nz - 1 && li + 1 < kTileW && lj + 1 < kTileW) {  // shear stress
+                double dvzdr = (n3[c] - ovz[c]) * s.idr;
+                if (i >= s.fRh) dvzdr += damp(kVzR, e, s.aRh, s.bRh, i, dvzdr);
+                double dvrdz = (n4[c] - ovr[c]) * s.idz;
+                if (j >= s.fZh) dvrdz += damp(kVrZ, e, s.aZh, s.bZh, j, dvrdz);
+                const double g = muZ[c] * (dvzdr + dvrdz);
+                orz[c] += s.dt * (LOSSY ? g + relax(s, &m[c][3], g) : g);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < kOwn; c++) {
+            const int e = ((threadIdx.x >> 5) + 16 * c) * kTileW + li;
+            trr[e] = orr[c];
+            tqq[e] = oqq[c];
+            tzz[e] = ozz[c];
+            trz[e] = orz[c];
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int c = 0; c < kOwn; c++) {
+        const int lj = (threadIdx.x >> 5) + 16 * c, e = lj * kTileW + li, j = gz + lj;
+        if (li < t.S || li >= t.S + tw || lj < t.S || lj >= t.S + tw || i >= s.nr || j >= s.nz) continue;
+        const size_t k = (size_t)j * s.nr + i;
+        t.out[kVr][k] = ovr[c];
+        t.out[kVz][k] = ovz[c];
+        t.out[kTrr][k] = orr[c];
+        t.out[kTqq][k] = oqq[c];
+        t.out[kTzz][k] = ozz[c];
+        t.out[kTrz][k] = orz[c];
+#pragma unroll
+        for (int f = 0; f < 4; f++)
+            if (LOSSY) t.out[kRrr + f][k] = m[c][f];
+#pragma unroll
+        for (int f = 0; f < 8; f++)
+            if (radial_psi[f] ? damp_r : damp_z) t.out[kTrrR + f][k] = psi[f * kTileCells + e];
+    }
+}
+
+// Steps per launch: the fewest estimated microseconds a step. A launch takes
+// about 8 us for its window's loads and stores and 2.1 per step (fitted on one
+// wave of tiles, S = 2 to 8), times its waves of one tile per SM of 148. On
+// 281 x 201 cells S = 2, 3, 4, 5, 6 took 6.3, 4.6, 4.2, 4.2, 5.9 us a step, on 6.1
+// million cells 223, 208, 209, 228, 259; one launch per phase 13.8 and 322.
+int tile_steps(int nr, int nz) {
+    int best = 1;
+    double least = INFINITY;
+    for (int S = 1; S <= kMaxTileSteps; S++) {
+        const double tw = kTileW - 2 * S, tiles = ceil(nr / tw) * ceil(nz / tw);
+        const double cost = ceil(tiles / 148) * (8.0 + 2.1 * S) / S;
+        if (cost < least) {
+            least = cost;
+            best = S;
+        }
+    }
+    return best;
 }
 
 // Block maxima of |vz| and |vr| (NaN propagates as NaN).
@@ -376,18 +648,21 @@ int gfk_fdtd_run(gfk_ctx* ctx, const gfk_fdtd_model* md, const double* force, in
     std::vector<void*> owned;
     auto dev = [&](size_t bytes) -> void* {
         void* p = nullptr;
-        if (cudaMallocAsync(&p, std::max<size_t>(bytes, 8), s) != cudaSuccess) return nullptr;
+        if (cudaMallocAsync(&p, std::max<size_t>(bytes, 8), s) != cudaSuccess) p = nullptr;
         owned.push_back(p);
-        cudaMemsetAsync(p, 0, std::max<size_t>(bytes, 8), s);
         return p;
     };
-    auto up = [&](const std::vector<double>& v) -> double* {
-        double* p = static_cast<double*>(dev(v.size() * 8));
-        if (p) cudaMemcpyAsync(p, v.data(), v.size() * 8, cudaMemcpyHostToDevice, s);
-        return p;
+    // the constants go up in one copy, once all of them are known
+    std::vector<double> consts;
+    std::vector<std::pair<const double**, size_t>> places;
+    auto up = [&](const std::vector<double>& v, const double** where) {
+        places.push_back({where, consts.size()});
+        consts.insert(consts.end(), v.begin(), v.end());
+        consts.resize((consts.size() + 31) / 32 * 32, 0.0);
     };
     auto cleanup = [&]() {
-        for (void* p : owned) cudaFreeAsync(p, s);
+        for (void* p : owned)
+            if (p) cudaFreeAsync(p, s);
         cudaStreamSynchronize(s);
     };
     gfk::fdtd::Args a{};
@@ -415,34 +690,59 @@ int gfk_fdtd_run(gfk_ctx* ctx, const gfk_fdtd_model* md, const double* force, in
     }
     a.idr = 1.0 / h;
     a.idz = 1.0 / h;
-    a.dt_rho = up(dtr);
-    a.dt_rhoZ = up(dtrz);
-    a.ir_half = up(irh);
-    a.ir_int = up(iri);
-    a.rho = up(rho);
-    a.lamU = up(lamU);
-    a.muU = up(muU);
-    a.rhoZ = up(rhoZ);
-    a.muZ = up(muZ);
-    a.aRi = up(pRi.a);
-    a.bRi = up(pRi.b);
-    a.aRh = up(pRh.a);
-    a.bRh = up(pRh.b);
-    a.aZi = up(pZi.a);
-    a.bZi = up(pZi.b);
-    a.aZh = up(pZh.a);
-    a.bZh = up(pZh.b);
+    up(dtr, &a.dt_rho);
+    up(dtrz, &a.dt_rhoZ);
+    up(irh, &a.ir_half);
+    up(iri, &a.ir_int);
+    up(rho, &a.rho);
+    up(lamU, &a.lamU);
+    up(muU, &a.muU);
+    up(rhoZ, &a.rhoZ);
+    up(muZ, &a.muZ);
+    up(pRi.a, &a.aRi);
+    up(pRi.b, &a.bRi);
+    up(pRh.a, &a.aRh);
+    up(pRh.b, &a.bRh);
+    up(pZi.a, &a.aZi);
+    up(pZi.b, &a.bZi);
+    up(pZh.a, &a.aZh);
+    up(pZh.b, &a.bZh);
     a.fRi = pRi.first;
     a.fRh = pRh.first;
     a.fZi = pZi.first;
     a.fZh = pZh.first;
-    double** fields[] = {&a.vr, &a.vz, &a.trr, &a.tqq, &a.tzz, &a.trz, &a.psiTrrR, &a.psiTrzZ, &a.psiTrzR,
-                         &a.psiTzzZ, &a.psiVrR, &a.psiVzZ, &a.psiVzR, &a.psiVrZ};
-    for (double** f : fields) *f = static_cast<double*>(dev(n * 8));
-    if (a.lossy) {
-        double** mem[] = {&a.rrr, &a.rqq, &a.rzz, &a.rrz};
-        for (double** f : mem) *f = static_cast<double*>(dev(n * 8));
+    // in the order of the kernel's field enumeration
+    double** fields[] = {&a.vr, &a.vz, &a.trr, &a.tqq, &a.tzz, &a.trz, &a.rrr, &a.rqq, &a.rzz, &a.rrz, &a.psiTrrR,
+                         &a.psiTrzZ, &a.psiTrzR, &a.psiTzzZ, &a.psiVrR, &a.psiVzZ, &a.psiVzR, &a.psiVrZ};
+    static_assert(sizeof fields / sizeof fields[0] == gfk::fdtd::kFields, "fields");
+    auto has = [&](int f) { return a.lossy || f < gfk::fdtd::kRrr || f > gfk::fdtd::kRrz; };
+    const int nfield = gfk::fdtd::kFields - (a.lossy ? 0 : 4);
+    // two copies of the fields, where they take at most half of what is free
+    // (asked only for large grids: the query takes up to a millisecond)
+    gfk::fdtd::Tiles tl{};
+    size_t mem_free = 0, mem_all = 0;
+    const bool fits = 2 * n * 8 * nfield <= (size_t(1) << 30) ||
+                      (cudaMemGetInfo(&mem_free, &mem_all) == cudaSuccess && 2 * n * 8 * nfield <= mem_free / 2);
+    const bool tiled = fits &&
+                       cudaFuncSetAttribute(a.lossy ? gfk::fdtd::k_tiles<true> : gfk::fdtd::k_tiles<false>,
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            gfk::fdtd::kTileSmem) == cudaSuccess;
+    std::vector<double> fpad(force, force + std::max(0, std::min(nforce, steps + 1)));
+    fpad.resize((size_t)steps + 1, 0.0);
+    const size_t copy = (n * 8 + 255) / 256 * 256, all = (tiled ? 2 : 1) * nfield * copy;
+    unsigned char* slab = static_cast<unsigned char*>(dev(all));
+    for (int f = 0, at = 0; slab && f < gfk::fdtd::kFields; f++)
+        if (has(f)) {
+            *fields[f] = reinterpret_cast<double*>(slab + at * copy);
+            tl.in[f] = *fields[f];
+            if (tiled) tl.out[f] = reinterpret_cast<double*>(slab + (nfield + at) * copy);
+            at++;
+        }
+    if (tiled) {
+        up(fpad, &tl.force);
+        tl.S = gfk::fdtd::tile_steps(nr, nz);
     }
+    double* d_consts = static_cast<double*>(dev(consts.size() * 8));
     int* d_cols = static_cast<int*>(dev(cols.size() * sizeof(int)));
     double* d_traces = static_cast<double*>(dev((size_t)std::max(nrcv, 1) * steps * 8));
     const int nblk = 296;
@@ -452,22 +752,50 @@ int gfk_fdtd_run(gfk_ctx* ctx, const gfk_fdtd_model* md, const double* force, in
             cleanup();
             return ffail(ctx, GFK_ENOMEM, "fdtd: device allocation failed");
         }
+    for (auto& [where, at] : places) *where = d_consts + at;
+    cudaMemsetAsync(slab, 0, all, s);
+    cudaMemsetAsync(d_traces, 0, (size_t)std::max(nrcv, 1) * steps * 8, s);
+    cudaMemcpyAsync(d_consts, consts.data(), consts.size() * 8, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(d_cols, cols.data(), cols.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     a.cols = d_cols;
     a.nrcv = nrcv;
     a.steps = steps;
     a.traces = d_traces;
 
-    auto force_at = [&](int i) { return (i < 0 || i >= nforce) ? 0.0 : force[i]; };
     const dim3 blk(32, 8), grd((nr + 31) / 32, (nz + 7) / 8);
     double peak = 0;
     std::vector<double> mx(nblk);
-    for (int step = 0; step < steps; step++) {  // fdtd.go:142-147, run.go:98-121
-        gfk::fdtd::k_velocities<<<grd, blk, 0, s>>>(a, -force_at(step) / a.src_area);
-        gfk::fdtd::k_stresses<<<grd, blk, 0, s>>>(a, (force_at(step + 1) - force_at(step)) / g.dt, step);
-        ctx->launches += 2;
-        if (step % 256 == 0) {
-            gfk::fdtd::k_maxspeed<<<nblk, 256, 0, s>>>(a.vz, a.vr, (long long)n, d_max);
+    for (int step = 0; step < steps;) {  // fdtd.go:142-147, run.go:98-121
+        // up to the next step whose speeds are checked (every 256th), at most S
+        int take = 1;
+        const double *vz = a.vz, *vr = a.vr;
+        if (tiled) {
+            take = std::min({tl.S, steps - step, step == 0 ? 1 : 256 - (step - 1) % 256});
+            tl.n = take;
+            tl.step0 = step;
+            const int tw = gfk::fdtd::kTileW - 2 * tl.S;
+            const dim3 tiles((nr + tw - 1) / tw, (nz + tw - 1) / tw);
+            if (a.lossy)
+                gfk::fdtd::k_tiles<true><<<tiles, gfk::fdtd::kTileThreads, gfk::fdtd::kTileSmem, s>>>(a, tl);
+            else
+                gfk::fdtd::k_tiles<false><<<tiles, gfk::fdtd::kTileThreads, gfk::fdtd::kTileSmem, s>>>(a, tl);
+            ctx->launches++;
+            for (int f = 0; f < gfk::fdtd::kFields; f++) {
+                double* o = tl.out[f];
+                tl.out[f] = const_cast<double*>(tl.in[f]);
+                tl.in[f] = o;
+            }
+            vz = tl.in[gfk::fdtd::kVz];
+            vr = tl.in[gfk::fdtd::kVr];
+        } else {
+            gfk::fdtd::k_velocities<<<grd, blk, 0, s>>>(a, -fpad[step] / a.src_area);
+            gfk::fdtd::k_stresses<<<grd, blk, 0, s>>>(a, (fpad[step + 1] - fpad[step]) / g.dt, step);
+            ctx->launches += 2;
+        }
+        step += take;
+        const int done = step - 1;
+        if (done % 256 == 0) {
+            gfk::fdtd::k_maxspeed<<<nblk, 256, 0, s>>>(vz, vr, (long long)n, d_max);
             ctx->launches++;
             if (cudaMemcpyAsync(mx.data(), d_max, nblk * 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                 cudaStreamSynchronize(s) != cudaSuccess) {
@@ -484,7 +812,7 @@ int gfk_fdtd_run(gfk_ctx* ctx, const gfk_fdtd_model* md, const double* force, in
             if (bad) {
                 cleanup();
                 char buf[96];
-                snprintf(buf, sizeof buf, "fdtd: diverged at step %d of %d", step, steps);
+                snprintf(buf, sizeof buf, "fdtd: diverged at step %d of %d", done, steps);
                 return ffail(ctx, GFK_ENONFINITE, buf);
             }
         }

@@ -74,8 +74,8 @@ class Sim:
         self.stack, self.sls, self.fref = stack, sls or SLS(), ref_freq
         h = spacing
         self.h, self.max_range, self.depth = h, max_range, depth
-        self.nr = int(round(max_range / h)) + 1 + pml_cells
-        self.nz = int(round(depth / h)) + 1 + pml_cells
+        self.nr = int(math.floor(max_range / h + 0.5)) + 1 + pml_cells
+        self.nz = int(math.floor(depth / h + 0.5)) + 1 + pml_cells
         lossy = self.sls.lossy()
         vmax = 0.0
         for l in stack:
