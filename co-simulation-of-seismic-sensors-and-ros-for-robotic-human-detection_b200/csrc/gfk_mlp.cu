@@ -16,11 +16,12 @@
 // writes W and W^T. The kernel shape is the wavenumber-sum kernel's: one
 // 128 x 128 tile per CTA, warp 0 TMA, warp 1 TMEM + MMA issue, warps 2-5
 // epilogue, SWIZZLE_64B tiles (32 BF16 = 64 bytes per row), 3-stage ring,
-// bounded waits. No cluster multicast.
+// bounded waits. Inference has a kernel of its own, k_layer_infer. No load is multicast.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <math_constants.h>
 
+#include <algorithm>
 #include <atomic>
 #include <utility>
 
@@ -46,8 +47,8 @@ constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + BN * 4;
 constexpr int kTileLd = BN + 8;  // BF16 row pitch of the epilogue's staging tiles (272 bytes)
 static_assert(2 * BM * kTileLd * 2 <= STAGES * STAGE_BYTES, "staging tiles alias the pipeline stages");
 
-// Instruction descriptor: BF16 x BF16 -> F32, both K-major, M = 128, N = 128.
-__host__ __device__ inline uint32_t idesc_bf16_128x128() {
+// Instruction descriptor: BF16 x BF16 -> F32, both K-major.
+__host__ __device__ inline uint32_t idesc_bf16(int m, int n) {
     cute::UMMA::InstrDescriptor id;
     id.desc_ = 0;
     id.c_format_ = 1;  // F32
@@ -55,8 +56,8 @@ __host__ __device__ inline uint32_t idesc_bf16_128x128() {
     id.b_format_ = 1;
     id.a_major_ = 0;   // K-major
     id.b_major_ = 0;
-    id.n_dim_ = BN >> 3;
-    id.m_dim_ = BM >> 4;
+    id.n_dim_ = n >> 3;
+    id.m_dim_ = m >> 4;
     return id.desc_;
 }
 
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(THREADS, 2)
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = idesc_bf16_128x128();
+            const uint32_t idesc = idesc_bf16(BM, BN);
             uint32_t acc = 0;
             for (int kb = 0; kb < nkb; kb++) {
                 const int st = kb % STAGES;
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(THREADS, 2)
         // BF16 results go to a shared-memory tile (the pipeline stages are free
         // once every MMA has completed), FP32 gradient partials straight out
         // the tile's bias columns, read once while the MMAs run
-        if (MODE == kFwdTrain || MODE == kFwdInfer) {
+        if (MODE == kFwdTrain) {
             bias_s[threadIdx.x - 64] = a.bias[n0 + threadIdx.x - 64];
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
@@ -241,14 +242,14 @@ __global__ void __launch_bounds__(THREADS, 2)
                 continue;
             }
             float y[32];
-            if (MODE == kFwdTrain || MODE == kFwdInfer) {
+            if (MODE == kFwdTrain) {
                 float zv[32];
 #pragma unroll
                 for (int c = 0; c < 32; c++) {
                     zv[c] = __uint_as_float(v[c]) + bias_s[j * 32 + c];
                     y[c] = zv[c] * sigmoid_(zv[c]);
                 }
-                if (MODE == kFwdTrain) {
+                {
                     uint4* zd = reinterpret_cast<uint4*>(tileZ + rl * kTileLd + j * 32);
 #pragma unroll
                     for (int c = 0; c < 4; c++)
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(THREADS, 2)
             if (MODE == kFwdTrain)
                 *reinterpret_cast<uint4*>(a.zout + g) = *reinterpret_cast<const uint4*>(tileZ + r * kTileLd + c8);
         }
-        if (MODE != kFwdInfer && a.outT) {
+        if (a.outT) {
             // 32 bytes (16 rows) of one transposed row per thread; lanes run
             // over columns, so the shared-memory column reads do not conflict
             for (int c = threadIdx.x; c < BN * (BM / 16); c += THREADS) {
@@ -310,6 +311,224 @@ __global__ void __launch_bounds__(THREADS, 2)
     if (threadIdx.x == 0 && *(volatile int*)abort_flag && a.status) atomicOr(a.status, kStTimeout);
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+}
+
+// ------------------------------------------------- inference layers --
+//
+// h = silu(x W^T + b) for many rows. A pair of CTAs on a pair of SMs keeps one
+// of the layer's 256-column slabs of weights in shared memory, half in each CTA
+// and the whole K extent (at most 512: 128 KB), and takes blocks of 256 rows,
+// which stream through a ring, again half in each: every SM computes 128 x 256
+// from 128 KB loaded. The leader of the pair issues the MMAs and its barriers
+// count both CTAs' loads. The accumulator is double-buffered in all 512 columns of
+// TMEM, so a tile's epilogue runs while the next one multiplies. Warp 0 loads,
+// warp 1 issues, warps 2-17 are the epilogue in two groups of 128 columns; a
+// group's 128 x 64 box of shared memory leaves by TMA. The order of K is
+// k_gemm's, and so are the results' bits.
+//
+// For 2^20 rows x 512 x 512 (2.1 GB at least, 0.32 ms of HBM, 0.35 ms of BF16):
+//   one tile per CTA (k_gemm), 32-wide K boxes          0.99 ms
+//   persistent, rows resident, weights streaming        0.93 ms  all SMs ask L2 for the same lines at a time
+//   128-column weights resident in each CTA alone       0.81 ms  256 KB loaded for 128 x 256, L2-bound
+//   pairs, 8 epilogue warps / 16                        0.60 / 0.58 ms
+// With K = 128 the loads are a quarter and it takes 0.43 ms: what is left is
+// the epilogue's chain (TMEM, exponentials, barriers, box) on 4 warps a scheduler.
+//
+// A producer stops only when a wait of its own has run out, a second after its
+// last load: nothing is in flight into a CTA that leaves.
+
+constexpr int kInfStages = 4;                       // row ring: 64 of K a stage
+constexpr int kInfKb = 8;                           // K blocks of 64 at most
+constexpr int kInfBlock = BM * 128;                 // 16 KB: 128 rows x 64 of K
+constexpr int kInfGroups = 2;                       // of eight epilogue warps, 128 columns each
+constexpr int kInfThreads = 64 + 256 * kInfGroups;
+constexpr int kInfBox = BM * 128;                   // output box: 128 rows x 64 columns
+constexpr int kInfN = 2 * BN;                       // columns of a pair's slab
+constexpr int kInfSmem = (kInfKb + kInfStages) * kInfBlock + kInfGroups * kInfBox + kInfN * 4 + 256 + 1024;
+static_assert(kInfSmem <= 227 * 1024, "shared memory per CTA");
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kInfThreads, 1)
+    k_layer_infer(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                  const __grid_constant__ CUtensorMap tmO, GemmArgs a) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* ring = smem + kInfKb * kInfBlock;
+    uint8_t* outs = ring + kInfStages * kInfBlock;  // one box per group
+    float* bias_s = reinterpret_cast<float*>(outs + kInfGroups * kInfBox);
+    uint64_t* w_full = reinterpret_cast<uint64_t*>(bias_s + kInfN);
+    uint64_t* a_full = w_full + 1;
+    uint64_t* a_empty = a_full + kInfStages;
+    uint64_t* acc_full = a_empty + kInfStages;
+    uint64_t* acc_empty = acc_full + 2;
+    uint64_t* drained = acc_empty + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile int* stop = abort_flag + 1;  // [kInfGroups] each epilogue group's common answer to it
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1;  // in the pair
+    const int nkb = a.K / BK, nslab = a.N / kInfN, nblock = (a.M + 2 * BM - 1) / (2 * BM);
+    const int n0 = ((blockIdx.x >> 1) % nslab) * kInfN;                             // the pair's columns
+    const int mb0 = (blockIdx.x >> 1) / nslab, mstep = (gridDim.x >> 1) / nslab;    // and row blocks
+    if (threadIdx.x == 0) {
+        mbar_init(w_full, 1);
+        for (int i = 0; i < kInfStages; i++) {
+            mbar_init(&a_full[i], 1);
+            mbar_init(&a_empty[i], 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_empty[i], 16 * kInfGroups);  // one arrival per epilogue warp of the pair
+        }
+        mbar_init(drained, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(2 * kInfN)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    dep_wait();  // the set-up above overlaps the previous kernel's tail
+    dep_release();
+    for (int n = threadIdx.x; n < kInfN; n += kInfThreads) bias_s[n] = a.bias[n0 + n];
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // the leader's barriers are there before the follower's loads count on them
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            const int row0 = rank * BM;
+            if (rank == 0) mbar_expect_tx(w_full, 2 * nkb * kInfBlock);
+            const uint32_t wbar = leader_addr(w_full);
+            for (int kb = 0; kb < nkb; kb++)
+                tma_load_2d_pair(smem + kb * kInfBlock, &tmB, wbar, kb * BK, n0 + row0);
+            int st = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int mb = mb0; mb < nblock && ok; mb += mstep)
+                for (int kb = 0; kb < nkb; kb++) {
+                    if (!mbar_wait(&a_empty[st], ph ^ 1)) {
+                        ok = false;
+                        break;
+                    }
+                    if (rank == 0) mbar_expect_tx(&a_full[st], 2 * kInfBlock);
+                    tma_load_2d_pair(ring + st * kInfBlock, &tmA, leader_addr(&a_full[st]), kb * BK, mb * 2 * BM + row0);
+                    if (++st == kInfStages) {
+                        st = 0;
+                        ph ^= 1;
+                    }
+                }
+            if (!ok) *abort_flag = 1;
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            const uint32_t idesc = idesc_bf16(2 * BM, kInfN);
+            int st = 0, tile = 0;
+            uint32_t ph = 0;
+            bool ok = leader_wait(w_full, 0);
+            for (int mb = mb0; mb < nblock && ok; mb += mstep, tile++) {
+                const int buf = tile & 1;
+                if (!leader_wait(&acc_empty[buf], ((tile >> 1) & 1) ^ 1) || *abort_flag) {
+                    ok = false;
+                    break;
+                }
+                for (int kb = 0; kb < nkb; kb++) {
+                    if (!leader_wait(&a_full[st], ph) || *abort_flag) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t ra = smem_u32(ring + st * kInfBlock), rb = smem_u32(smem + kb * kInfBlock);
+#pragma unroll
+                    for (int kk = 0; kk < BK / 16; kk++)  // K = 16 per instruction = 32 bytes of the row
+                        tc_mma_f16_pair(tmem + buf * kInfN, sdesc_k_sw128(ra + kk * 32), sdesc_k_sw128(rb + kk * 32),
+                                        idesc, (kb | kk) ? 1u : 0u);
+                    tc_commit_pair(&a_empty[st]);
+                    if (++st == kInfStages) {
+                        st = 0;
+                        ph ^= 1;
+                    }
+                }
+                if (ok) tc_commit_pair(&acc_full[buf]);
+            }
+            if (!ok) *abort_flag = 1;
+            tc_commit_pair(drained);  // every MMA issued above, before TMEM is freed
+        }
+    } else {
+        const int q = warp & 3, group = (warp - 2) >> 3, sub = ((warp - 2) >> 2) & 1;
+        const bool lead = ((warp - 2) & 7) == 0 && lane == 0;  // issues its group's stores
+        uint8_t* const box = outs + group * kInfBox;
+        const int rl = q * 32 + lane;
+        auto group_sync = [&] { asm volatile("bar.sync %0, 256;" ::"r"(1 + group) : "memory"); };
+        int tile = 0;
+        for (int mb = mb0; mb < nblock; mb += mstep, tile++) {
+            const int buf = tile & 1;
+            if (!mbar_wait(&acc_full[buf], (tile >> 1) & 1)) *abort_flag = 1;
+            __syncwarp();
+            tc_fence_after();
+            const uint32_t at = tmem + (static_cast<uint32_t>(q * 32) << 16) + buf * kInfN + group * BN + sub * 32;
+            const int row = (mb * 2 + rank) * BM;
+            bool run = true;
+#pragma unroll
+            for (int c = 0; c < 2; c++) {  // 64 columns at a time, 32 in each warp
+                uint32_t v[32];
+                tmem_ld32(at + c * 64, v);
+                tmem_wait_ld();
+                if (c == 1) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) leader_arrive(leader_addr(&acc_empty[buf]));
+                }
+                uint4 y4[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    float y[8];
+#pragma unroll
+                    for (int e = 0; e < 8; e++) {
+                        const float z = __uint_as_float(v[8 * j + e]) + bias_s[group * BN + c * 64 + sub * 32 + 8 * j + e];
+                        y[e] = z * sigmoid_(z);
+                    }
+                    y4[j] = make_uint4(pack2(y[0], y[1]), pack2(y[2], y[3]), pack2(y[4], y[5]), pack2(y[6], y[7]));
+                }
+                if (lead) {
+                    tma_store_wait_read();  // the box is free again
+                    stop[group] = *abort_flag;
+                }
+                group_sync();
+                // once a wait has run out the group stops together: the next write of
+                // stop[group] comes after the barrier below, when all have read it
+                if (stop[group]) {
+                    run = false;
+                    break;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    *reinterpret_cast<uint4*>(box + rl * 128 + (((sub * 4 + j) ^ (rl & 7)) << 4)) = y4[j];
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                group_sync();
+                if (lead && row < a.M) {  // an odd last block has rows in the leader only
+                    tma_store_2d(&tmO, box, n0 + group * BN + c * 64, row);
+                    tma_store_commit();
+                }
+            }
+            if (!run) break;
+        }
+        if (lead) tma_store_wait();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 32 && !mbar_wait(drained, 0)) *abort_flag = 1;
+    __syncthreads();
+    cluster_sync();  // neither CTA leaves while the other may still signal it or read its operands
+    tc_fence_after();
+    if (threadIdx.x == 0 && *abort_flag && a.status) atomicOr(a.status, kStTimeout);
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kInfN) : "memory");
 }
 
 // ----------------------------------------------------------------- batch --
@@ -958,16 +1177,16 @@ __global__ void __launch_bounds__(256) k_eval(const float* T, const float* label
 // ------------------------------------------------------------------ host --
 
 namespace {
-bool make_map_bf16(CUtensorMap* map, const bf16* base, int rows, int K) {
+bool make_map_bf16(CUtensorMap* map, const bf16* base, int rows, int K, bool wide = false) {
     auto fn = encode_fn();
     if (!fn) return false;
     cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    cuuint32_t box[2] = {(cuuint32_t)BKE, (cuuint32_t)BM};
+    cuuint32_t box[2] = {(cuuint32_t)(wide ? BK : BKE), (cuuint32_t)BM};
     cuuint32_t estr[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+              CU_TENSOR_MAP_INTERLEAVE_NONE, wide ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int MODE>
@@ -989,8 +1208,8 @@ void launch_mode(cudaStream_t s, const CUtensorMap& ta, const CUtensorMap& tb, d
 
 int prepare_gemm() {
     static std::atomic<bool> done{false};
-    if (!done.load(std::memory_order_relaxed) && set_attr<kFwdTrain>() && set_attr<kFwdInfer>() &&
-        set_attr<kBwdData>() && set_attr<kWgrad>())
+    if (!done.load(std::memory_order_relaxed) && set_attr<kFwdTrain>() && set_attr<kBwdData>() && set_attr<kWgrad>() &&
+        cudaFuncSetAttribute(k_layer_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kInfSmem) == cudaSuccess)
         done.store(true, std::memory_order_relaxed);
     return done.load(std::memory_order_relaxed) ? 0 : 3;
 }
@@ -1008,7 +1227,21 @@ int launch_gemm(cudaStream_t s, int mode, const bf16* A, const bf16* B, int rows
     const dim3 grid(rowsB / BN, rowsA / BM, splits);
     switch (mode) {
         case kFwdTrain: launch_mode<kFwdTrain>(s, ta, tb, grid, a); return 0;
-        case kFwdInfer: launch_mode<kFwdInfer>(s, ta, tb, grid, a); return 0;
+        case kFwdInfer: {
+            if (splits != 1 || a.K / BK > kInfKb || a.N % kInfN) return 1;
+            int dev = 0, sms = 0;
+            if (cudaGetDevice(&dev) != cudaSuccess ||
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+                return 3;
+            CUtensorMap to;
+            if (!make_map_bf16(&ta, A, rowsA, ktotal, true) || !make_map_bf16(&tb, B, rowsB, ktotal, true) ||
+                !make_map_bf16(&to, a.out, rowsA, rowsB, true))
+                return 2;
+            const int slabs = rowsB / kInfN;  // a pair of CTAs per pair of SMs, as many for each slab
+            const int pairs = slabs * std::max(1, std::min(sms / 2 / slabs, (rowsA + 2 * BM - 1) / (2 * BM)));
+            launch_dep(k_layer_infer, dim3(2 * pairs), dim3(kInfThreads), kInfSmem, s, ta, tb, to, a);
+            return 0;
+        }
         case kBwdData: launch_mode<kBwdData>(s, ta, tb, grid, a); return 0;
         case kWgrad: launch_mode<kWgrad>(s, ta, tb, grid, a); return 0;
     }
