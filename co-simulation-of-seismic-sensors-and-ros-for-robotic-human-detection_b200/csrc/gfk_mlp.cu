@@ -587,6 +587,24 @@ __device__ __forceinline__ float feature(int j, const float* sf, const PointScal
     return (j & 1) ? cs : sn;
 }
 
+// Features j and j + 1, j even: a sine and cosine share their argument and one call.
+__device__ __forceinline__ void feature_pair(int j, const float* sf, const PointScalars& p, const float* four, float& v0,
+                                             float& v1) {
+    if ((j >= kTimeFeat && j < kLogTimeFeat) || j >= kFourierFeat) {
+        const int f = (j - kFourierFeat) >> 1;
+        const float arg = j < kLogTimeFeat ? 2.0f * (p.f * sf[kScalars + ((j - kTimeFeat) >> 1)])
+                                           : 2.0f * (four[2 * f] * p.ur + four[2 * f + 1] * p.uf);
+        sincospif(arg, &v0, &v1);
+    } else {
+        v0 = feature(j, sf, p, four);
+        v1 = feature(j + 1, sf, p, four);
+    }
+}
+static_assert(kTimeFeat % 2 == 0 && kLogTimeFeat % 2 == 0 && kFourierFeat % 2 == 0, "features come in pairs");
+
+// The step's counter and rates. The batch draws with the counter's next value, so
+// this one-thread kernel (two FP64 powers) runs beside the last weight
+// gradients, before the loss history and Adam, which read what it writes.
 __global__ void k_step_begin(TrainScalars* ts) {
     dep_wait();
     dep_release();
@@ -604,28 +622,36 @@ __global__ void k_step_begin(TrainScalars* ts) {
     ts->bc2 = static_cast<float>(1.0 - pow(static_cast<double>(ts->beta2), static_cast<double>(t)));
 }
 
-// kBatchRows samples per block: one thread per sample draws the cell and builds
-// its scalars and targets, then one thread per feature fills the rows. Small
+// kBatchRows samples per block. A lane per sample of one warp draws the cell and
+// gathers its targets while the lanes of another form the samples' scalars (FP64
+// logarithms); then a thread fills a pair of features of four samples. Small
 // blocks keep many of them resident, so the dependent gathers (soil, cell,
-// label) of different blocks overlap.
+// label) of different blocks overlap. (One warp doing both and a thread per
+// feature walking 16 samples: 16.1 us for 8192 samples; 9.0 us here, cold.)
 constexpr int kBatchRows = 16;
-__global__ void __launch_bounds__(kIn) k_batch(BatchArgs a) {
+constexpr int kBatchThreads = 256;
+__global__ void __launch_bounds__(kBatchThreads) k_batch(BatchArgs a) {
     dep_wait();
     dep_release();
-    __shared__ bf16 tile[kBatchRows][kIn + 2];
+    __shared__ uint32_t tile[kBatchRows][kIn / 2 + 1];  // pairs of BF16
     __shared__ PointScalars ps[kBatchRows];
     __shared__ int soil_of[kBatchRows];
-    const long long t = a.ts->step;
+    const long long t = a.ts->step + 1;
     const int b0 = blockIdx.x * kBatchRows;
-    const int j = threadIdx.x;
-    if (j < kBatchRows) {
-        const int b = b0 + j;
-        const unsigned long long h = mix64(a.seed ^ mix64(static_cast<unsigned long long>(t) * a.B + b));
-        const int soil = a.train[pick(h, a.ntrain)];
+    const int tid = threadIdx.x, sample = tid & 31;
+    unsigned long long h = 0;
+    int ir = 0, jf = 0;
+    if (tid < 64 && sample < kBatchRows) {
+        h = mix64(a.seed ^ mix64(static_cast<unsigned long long>(t) * a.B + b0 + sample));
         const unsigned long long h2 = mix64(h);
-        const int ir = a.ir0 + pick(h2, a.nir), jf = pick(h2 >> 32, a.nf);
-        ps[j] = point_scalars(a.ranges[ir], a.freqs[jf], a.dom);
-        soil_of[j] = soil;
+        ir = a.ir0 + pick(h2, a.nir);
+        jf = pick(h2 >> 32, a.nf);
+    }
+    if (tid >= 32 && tid < 32 + kBatchRows) ps[sample] = point_scalars(a.ranges[ir], a.freqs[jf], a.dom);
+    if (tid < kBatchRows) {
+        const int b = b0 + sample;
+        const int soil = a.train[pick(h, a.ntrain)];
+        soil_of[sample] = soil;
         const float* L = a.labels + (((size_t)soil * a.nr + ir) * a.nf + jf) * 2;
         const bool ph = !isnan(L[1]);
         a.Y[2 * b] = (L[0] - a.y_mean0) / a.y_std0;
@@ -646,143 +672,180 @@ __global__ void __launch_bounds__(kIn) k_batch(BatchArgs a) {
         a.C[2 * b + 1] = c1;
     }
     __syncthreads();
-    for (int i = 0; i < kBatchRows; i++)
-        tile[i][j] = __float2bfloat16_rn(feature(j, a.soilfeat + (size_t)soil_of[i] * kSoilStride, ps[i], a.fourier));
-    __syncthreads();
-    for (int i = 0; i < kBatchRows; i++) a.X[(size_t)(b0 + i) * kIn + j] = tile[i][j];
-    // X^T: thread j writes its feature's kBatchRows consecutive samples
-    uint32_t w[kBatchRows / 2];
+    const int pair = tid & 63;
 #pragma unroll
-    for (int i = 0; i < kBatchRows / 2; i++) {
-        __nv_bfloat162 v;
-        v.x = tile[2 * i][j];
-        v.y = tile[2 * i + 1][j];
-        w[i] = *reinterpret_cast<uint32_t*>(&v);
+    for (int i = tid >> 6; i < kBatchRows; i += kBatchThreads / 64) {
+        float v0, v1;
+        feature_pair(2 * pair, a.soilfeat + (size_t)soil_of[i] * kSoilStride, ps[i], a.fourier, v0, v1);
+        const uint32_t v = pack2(v0, v1);
+        tile[i][pair] = v;
+        *reinterpret_cast<uint32_t*>(a.X + (size_t)(b0 + i) * kIn + 2 * pair) = v;
     }
-    uint4* d = reinterpret_cast<uint4*>(a.XT + (size_t)j * a.B + b0);
+    __syncthreads();
+    // X^T: a thread writes 8 consecutive samples of its feature
+    const int j = tid & (kIn - 1), half = tid / kIn;
+    uint32_t w[4];
 #pragma unroll
-    for (int i = 0; i < kBatchRows / 8; i++) d[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+    for (int i = 0; i < 4; i++) {
+        const uint32_t lo = tile[8 * half + 2 * i][j >> 1], hi = tile[8 * half + 2 * i + 1][j >> 1];
+        w[i] = __byte_perm(lo, hi, (j & 1) ? 0x7632 : 0x5410);
+    }
+    *reinterpret_cast<uint4*>(a.XT + (size_t)j * a.B + b0 + 8 * half) = make_uint4(w[0], w[1], w[2], w[3]);
 }
+static_assert(kBatchRows == 16 && kBatchThreads == 2 * kIn, "two groups of 8 samples");
 
 // ------------------------------------------------------------------ head --
 
-// 8 warps x 4 rows; lane owns columns u*256 + lane*8 + e (u = 0, 1; e < 8).
-__global__ void __launch_bounds__(256) k_head_train(const bf16* __restrict__ H, const bf16* __restrict__ Z,
-                                                    const float* __restrict__ W6, const float* __restrict__ b6,
-                                                    const float* __restrict__ Y, const float* __restrict__ Cw, int B,
-                                                    bf16* __restrict__ dZ, bf16* __restrict__ dZT,
-                                                    float* __restrict__ gpart, float* __restrict__ lpart) {
+// 8 warps x 4 rows; lane owns columns u*256 + lane*8 + e (u = 0, 1; e < 8). A
+// warp asks for its four rows of H and Z at once and carries the four dot
+// products together, then walks the columns with the rows inside, and the
+// warps' dW6 parts meet in shared memory in one step, added in warp order. (A row
+// after the other, a load and a shuffle chain each, and one barrier per warp for
+// the parts: 27.7 us for 8192 rows, 34 MB; 13.1 us here, cold.)
+struct HeadShared {
+    bf16 tile[kHeadRows][kWidth + 8];
+    float part[8][2 * kWidth];
+};
+__global__ void __launch_bounds__(256, 2) k_head_train(const bf16* __restrict__ H, const bf16* __restrict__ Z,
+                                                       const float* __restrict__ W6, const float* __restrict__ b6,
+                                                       const float* __restrict__ Y, const float* __restrict__ Cw, int B,
+                                                       bf16* __restrict__ dZ, bf16* __restrict__ dZT,
+                                                       float* __restrict__ gpart, float* __restrict__ lpart) {
     dep_wait();
     dep_release();
-    __shared__ __align__(16) bf16 tile[kHeadRows][kWidth + 8];
-    __shared__ float red[2 * kWidth + 2];
-    __shared__ float lred[8][4];
+    extern __shared__ __align__(16) uint8_t head_raw[];
+    HeadShared& sm = *reinterpret_cast<HeadShared*>(head_raw);
+    __shared__ float lred[8][6];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = blockIdx.x * kHeadRows;
-    float w0[16], w1[16], g0[16], g1[16];
+    const int r0 = blockIdx.x * kHeadRows, row = r0 + warp * 4;
+    uint4 hq[4][2], zq[4][2];
+    float2 yt[4], ct[4];
 #pragma unroll
-    for (int u = 0; u < 2; u++)
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            const int c = u * 256 + lane * 8 + e;
-            w0[u * 8 + e] = W6[c];
-            w1[u * 8 + e] = W6[kWidth + c];
-            g0[u * 8 + e] = 0.0f;
-            g1[u * 8 + e] = 0.0f;
-        }
-    float l0 = 0.0f, l1 = 0.0f, sc0 = 0.0f, sc1 = 0.0f, ds0 = 0.0f, ds1 = 0.0f;
-    for (int t = 0; t < 4; t++) {
-        const int rl = warp * 4 + t, row = r0 + rl;
-        float h[16], z[16];
+    for (int t = 0; t < 4; t++)
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-            unpack8(*reinterpret_cast<const uint4*>(H + (size_t)row * kWidth + u * 256 + lane * 8), h + 8 * u);
-            unpack8(*reinterpret_cast<const uint4*>(Z + (size_t)row * kWidth + u * 256 + lane * 8), z + 8 * u);
-        }
-        float y0 = 0.0f, y1 = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            y0 = fmaf(h[i], w0[i], y0);
-            y1 = fmaf(h[i], w1[i], y1);
+            hq[t][u] = *reinterpret_cast<const uint4*>(H + (size_t)(row + t) * kWidth + u * 256 + lane * 8);
+            zq[t][u] = *reinterpret_cast<const uint4*>(Z + (size_t)(row + t) * kWidth + u * 256 + lane * 8);
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            y0 += __shfl_xor_sync(0xffffffffu, y0, o);
-            y1 += __shfl_xor_sync(0xffffffffu, y1, o);
+    for (int t = 0; t < 4; t++) {
+        yt[t] = *reinterpret_cast<const float2*>(Y + 2 * (row + t));
+        ct[t] = *reinterpret_cast<const float2*>(Cw + 2 * (row + t));
+    }
+    auto load8 = [](const float* src, float (&w)[8]) {
+        const float4 x = *reinterpret_cast<const float4*>(src), y = *reinterpret_cast<const float4*>(src + 4);
+        w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w, w[4] = y.x, w[5] = y.y, w[6] = y.z, w[7] = y.w;
+    };
+    float y0[4] = {}, y1[4] = {};
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        float w0[8], w1[8];
+        load8(W6 + u * 256 + lane * 8, w0);
+        load8(W6 + kWidth + u * 256 + lane * 8, w1);
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            float h[8];
+            unpack8(hq[t][u], h);
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                y0[t] = fmaf(h[e], w0[e], y0[t]);
+                y1[t] = fmaf(h[e], w1[e], y1[t]);
+            }
         }
-        y0 += b6[0];
-        y1 += b6[1];
-        const float t0 = Y[2 * row], t1 = Y[2 * row + 1];
-        const float c0 = Cw[2 * row], c1 = Cw[2 * row + 1];
-        const bool ph = !isnan(t1) && c1 > 0.0f;
-        const float e0 = y0 - t0, e1 = ph ? y1 - t1 : 0.0f;
-        const float d0 = 2.0f * c0 * e0 / B, d1 = ph ? 2.0f * c1 * e1 / B : 0.0f;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            y0[t] += __shfl_xor_sync(0xffffffffu, y0[t], o);
+            y1[t] += __shfl_xor_sync(0xffffffffu, y1[t], o);
+        }
+    float l0 = 0.0f, l1 = 0.0f, sc0 = 0.0f, sc1 = 0.0f, ds0 = 0.0f, ds1 = 0.0f;
+    float d0[4], d1[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        const float c0 = ct[t].x, c1 = ct[t].y;
+        const bool ph = !isnan(yt[t].y) && c1 > 0.0f;
+        const float e0 = (y0[t] + b6[0]) - yt[t].x, e1 = ph ? (y1[t] + b6[1]) - yt[t].y : 0.0f;
+        d0[t] = 2.0f * c0 * e0 / B;
+        d1[t] = ph ? 2.0f * c1 * e1 / B : 0.0f;
         l0 += c0 * e0 * e0;
         l1 += ph ? c1 * e1 * e1 : 0.0f;
         sc0 += c0;
         sc1 += ph ? c1 : 0.0f;
-        ds0 += d0;
-        ds1 += d1;
-        float dz[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            g0[i] = fmaf(d0, h[i], g0[i]);
-            g1[i] = fmaf(d1, h[i], g1[i]);
-            const float dh = d0 * w0[i] + d1 * w1[i];
-            const float sg = sigmoid_(z[i]);
-            dz[i] = dh * (sg * (1.0f + z[i] * (1.0f - sg)));
-        }
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const uint4 pk = make_uint4(pack2(dz[8 * u], dz[8 * u + 1]), pack2(dz[8 * u + 2], dz[8 * u + 3]),
-                                        pack2(dz[8 * u + 4], dz[8 * u + 5]), pack2(dz[8 * u + 6], dz[8 * u + 7]));
-            *reinterpret_cast<uint4*>(dZ + (size_t)row * kWidth + u * 256 + lane * 8) = pk;
-            *reinterpret_cast<uint4*>(&tile[rl][u * 256 + lane * 8]) = pk;
-        }
+        ds0 += d0[t];
+        ds1 += d1[t];
     }
-    // deterministic cross-warp sum of the dW6 / db6 contributions
-    for (int w = 0; w < 8; w++) {
-        if (warp == w) {
+    if (lane == 0) {
+        lred[warp][0] = l0;
+        lred[warp][1] = l1;
+        lred[warp][2] = sc0;
+        lred[warp][3] = sc1;
+        lred[warp][4] = ds0;
+        lred[warp][5] = ds1;
+    }
+    // opaque: else the compiler keeps the first pass's 64 unpacked values and spills
 #pragma unroll
-            for (int u = 0; u < 2; u++)
+    for (int t = 0; t < 4; t++)
 #pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const int c = u * 256 + lane * 8 + e;
-                    red[c] = (w ? red[c] : 0.0f) + g0[u * 8 + e];
-                    red[kWidth + c] = (w ? red[kWidth + c] : 0.0f) + g1[u * 8 + e];
-                }
-            if (lane == 0) {
-                red[2 * kWidth] = (w ? red[2 * kWidth] : 0.0f) + ds0;
-                red[2 * kWidth + 1] = (w ? red[2 * kWidth + 1] : 0.0f) + ds1;
-                lred[w][0] = l0;
-                lred[w][1] = l1;
-                lred[w][2] = sc0;
-                lred[w][3] = sc1;
+        for (int u = 0; u < 2; u++)
+            asm volatile("" : "+r"(hq[t][u].x), "+r"(hq[t][u].y), "+r"(hq[t][u].z), "+r"(hq[t][u].w));
+    asm volatile("" : "+l"(W6));
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        float w0[8], w1[8], g0[8] = {}, g1[8] = {};
+        load8(W6 + u * 256 + lane * 8, w0);
+        load8(W6 + kWidth + u * 256 + lane * 8, w1);
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            float h[8], z[8], dz[8];
+            unpack8(hq[t][u], h);
+            unpack8(zq[t][u], z);
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                g0[e] = fmaf(d0[t], h[e], g0[e]);
+                g1[e] = fmaf(d1[t], h[e], g1[e]);
+                const float dh = d0[t] * w0[e] + d1[t] * w1[e];
+                const float sg = sigmoid_(z[e]);
+                dz[e] = dh * (sg * (1.0f + z[e] * (1.0f - sg)));
             }
+            const uint4 pk = make_uint4(pack2(dz[0], dz[1]), pack2(dz[2], dz[3]), pack2(dz[4], dz[5]),
+                                        pack2(dz[6], dz[7]));
+            *reinterpret_cast<uint4*>(dZ + (size_t)(row + t) * kWidth + u * 256 + lane * 8) = pk;
+            *reinterpret_cast<uint4*>(&sm.tile[warp * 4 + t][u * 256 + lane * 8]) = pk;
         }
-        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 8; k += 4) {
+            const int c = u * 256 + lane * 8 + k;
+            *reinterpret_cast<float4*>(&sm.part[warp][c]) = make_float4(g0[k], g0[k + 1], g0[k + 2], g0[k + 3]);
+            *reinterpret_cast<float4*>(&sm.part[warp][kWidth + c]) = make_float4(g1[k], g1[k + 1], g1[k + 2], g1[k + 3]);
+        }
     }
-    for (int i = threadIdx.x; i < kHeadStride; i += blockDim.x)
-        gpart[(size_t)blockIdx.x * kHeadStride + i] = i < 2 * kWidth + 2 ? red[i] : 0.0f;
-    if (threadIdx.x == 0) {
-        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        for (int w = 0; w < 8; w++)
-            for (int q = 0; q < 4; q++) s[q] += lred[w][q];
-        for (int q = 0; q < 4; q++) lpart[blockIdx.x * 4 + q] = s[q];
-    }
+    __syncthreads();
     // dZ^T: 32 consecutive rows of column c, 64 bytes per store group
     for (int c = threadIdx.x; c < kWidth; c += blockDim.x) {
         uint32_t w[16];
 #pragma unroll
         for (int i = 0; i < 16; i++) {
             __nv_bfloat162 v;
-            v.x = tile[2 * i][c];
-            v.y = tile[2 * i + 1][c];
+            v.x = sm.tile[2 * i][c];
+            v.y = sm.tile[2 * i + 1][c];
             w[i] = *reinterpret_cast<uint32_t*>(&v);
         }
         uint4* d = reinterpret_cast<uint4*>(dZT + (size_t)c * B + r0);
 #pragma unroll
         for (int i = 0; i < 4; i++) d[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+    }
+    for (int i = threadIdx.x; i < kHeadStride; i += blockDim.x) {
+        float v = 0.0f;
+        if (i < 2 * kWidth + 2)
+            for (int w = 0; w < 8; w++) v += i < 2 * kWidth ? sm.part[w][i] : lred[w][4 + i - 2 * kWidth];
+        gpart[(size_t)blockIdx.x * kHeadStride + i] = v;
+    }
+    if (threadIdx.x < 4) {
+        float v = 0.0f;
+        for (int w = 0; w < 8; w++) v += lred[w][threadIdx.x];
+        lpart[blockIdx.x * 4 + threadIdx.x] = v;
     }
 }
 
@@ -843,29 +906,118 @@ __device__ __forceinline__ float seg_grad(const AdamSeg& g, long long j) {
 }
 
 // AdamW (Loshchilov & Hutter 2019) on the FP32 master copy, gradients summed
-// from their partials in a fixed order; refreshes the BF16 copy W.
-__global__ void k_adam(AdamArgs a) {
-    dep_wait();
-    dep_release();
-    const AdamSeg g = a.dseg[blockIdx.y];
-    const long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (j >= g.n) return;
-    const long long i = g.off + j;
-    const float m0 = a.m[i], v0 = a.v[i];
-    float p = a.p[i];
-    const float grad = seg_grad(g, j);
-    const TrainScalars* ts = a.ts;
-    const float b1 = ts->beta1, b2 = ts->beta2;
+// from their partials in a fixed order; refreshes the BF16 copies W and W^T.
+__device__ __forceinline__ float adam_one(const AdamArgs& a, const TrainScalars& ts, long long i, float m0, float v0, float p,
+                                          float grad) {
+    const float b1 = ts.beta1, b2 = ts.beta2;
     const float m = b1 * m0 + (1.0f - b1) * grad;
     const float v = b2 * v0 + (1.0f - b2) * grad * grad;
     a.m[i] = m;
     a.v[i] = v;
-    p -= ts->lr * ((m / ts->bc1) / (sqrtf(v / ts->bc2) + a.eps) + a.weight_decay * p);
+    p -= ts.lr * ((m / ts.bc1) / (sqrtf(v / ts.bc2) + a.eps) + a.weight_decay * p);
     a.p[i] = p;
-    if (g.wb) g.wb[j] = __float2bfloat16_rn(p);
+    return p;
 }
 
-// W^T from W for every weight segment, 32 x 32 tiles through shared memory.
+// A block of 256 threads takes a 32 x 32 tile of a weight segment, whose W^T goes
+// out through shared memory; 256 parameters of a segment without copies; or 32
+// parameters of one with many partials (the head's 256): it loads 128 partials of each at
+// a time and a thread adds its parameter's in order. (One parameter per
+// thread everywhere and the transposes in a launch of their own: 30.3 + 6.6 us
+// for 1.1 M parameters, 36 MB of partials and 31 MB of state; 17.7 us here, cold.)
+constexpr int kAdamMany = 32;  // partials from which a block takes 32 parameters
+__host__ __device__ inline long long adam_items(const AdamSeg& g) {
+    return g.wb ? 1024 : g.nsrc > kAdamMany ? 32 : 256;
+}
+__global__ void __launch_bounds__(256) k_adam(AdamArgs a) {
+    dep_wait();
+    dep_release();
+    __shared__ union {
+        bf16 t[32][33];
+        float part[128][33];
+    } sm;
+    const AdamSeg g = a.dseg[blockIdx.y];
+    const long long j0 = blockIdx.x * adam_items(g);
+    if (j0 >= g.n) return;
+    const TrainScalars ts = *a.ts;
+    const int tid = threadIdx.x, x = tid & 31, y = tid >> 5;
+    if (g.wb) {
+        const int tiles = g.cols / 32, r0 = (blockIdx.x / tiles) * 32, c0 = (blockIdx.x % tiles) * 32;
+        float m[4], v[4], p[4], grad[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const long long i = g.off + (long long)(r0 + y + 8 * k) * g.cols + c0 + x;
+            m[k] = a.m[i];
+            v[k] = a.v[i];
+            p[k] = a.p[i];
+            grad[k] = 0.0f;
+        }
+        int q = 0;
+        for (; q + 4 <= g.nsrc; q += 4) {  // 16 loads in flight
+            float u[4][4];
+#pragma unroll
+            for (int w = 0; w < 4; w++)
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    u[w][k] = __ldg(g.src + (q + w) * g.stride + (long long)(r0 + y + 8 * k) * g.cols + c0 + x);
+#pragma unroll
+            for (int w = 0; w < 4; w++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) grad[k] += u[w][k];
+        }
+        for (; q < g.nsrc; q++)
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                grad[k] += __ldg(g.src + q * g.stride + (long long)(r0 + y + 8 * k) * g.cols + c0 + x);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const long long j = (long long)(r0 + y + 8 * k) * g.cols + c0 + x;
+            const bf16 w = __float2bfloat16_rn(adam_one(a, ts, g.off + j, m[k], v[k], p[k], grad[k]));
+            g.wb[j] = w;
+            sm.t[y + 8 * k][x] = w;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; k++) g.wt[(size_t)(c0 + y + 8 * k) * g.rows + r0 + x] = sm.t[x][y + 8 * k];
+        return;
+    }
+    if (g.nsrc <= kAdamMany) {
+        const long long j = j0 + tid;
+        if (j < g.n) adam_one(a, ts, g.off + j, a.m[g.off + j], a.v[g.off + j], a.p[g.off + j], seg_grad(g, j));
+        return;
+    }
+    const long long j = j0 + x, i = g.off + j;
+    float grad = 0.0f, m = 0.0f, v = 0.0f, p = 0.0f;
+    const bool own = y == 0 && j < g.n;
+    if (own) {
+        m = a.m[i];
+        v = a.v[i];
+        p = a.p[i];
+    }
+    for (int q0 = 0; q0 < g.nsrc; q0 += 128) {
+        const int nq = g.nsrc - q0 < 128 ? g.nsrc - q0 : 128;
+        if (j < g.n) {
+            float u[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) u[k] = y + 8 * k < nq ? __ldg(g.src + (q0 + y + 8 * k) * g.stride + j) : 0.0f;
+#pragma unroll
+            for (int k = 0; k < 16; k++) sm.part[y + 8 * k][x] = u[k];
+        }
+        __syncthreads();
+        if (own) {
+            int q = 0;
+            for (; q + 16 <= nq; q += 16)
+#pragma unroll
+                for (int k = 0; k < 16; k++) grad += sm.part[q + k][x];
+            for (; q < nq; q++) grad += sm.part[q][x];
+        }
+        __syncthreads();
+    }
+    if (own) adam_one(a, ts, i, m, v, p, grad);
+}
+
+// W^T from W for every weight segment (parameters set from outside), 32 x 32
+// tiles through shared memory.
 __global__ void k_transpose_w(AdamArgs a) {
     dep_wait();
     dep_release();
@@ -945,23 +1097,10 @@ __global__ void __launch_bounds__(kFeatThreads) k_features(FeatureArgs a, long l
         const long long q = q0 + i;
         if (q >= rows_padded) return;
         float v0 = 0.0f, v1 = 0.0f;
-        if (const float* sf = soil[i]) {
-            const int j = 2 * pair;
-            if ((j >= kTimeFeat && j < kLogTimeFeat) || j >= kFourierFeat) {
-                const int f = (j - kFourierFeat) >> 1;
-                const float arg = j < kLogTimeFeat ? 2.0f * (ps[i].f * sf[kScalars + ((j - kTimeFeat) >> 1)])
-                                                   : 2.0f * (a.fourier[2 * f] * ps[i].ur + a.fourier[2 * f + 1] * ps[i].uf);
-                sincospif(arg, &v0, &v1);
-            } else {
-                v0 = feature(j, sf, ps[i], a.fourier);
-                v1 = feature(j + 1, sf, ps[i], a.fourier);
-            }
-        }
+        if (const float* sf = soil[i]) feature_pair(2 * pair, sf, ps[i], a.fourier, v0, v1);
         *reinterpret_cast<uint32_t*>(a.X + q * kIn + 2 * pair) = pack2(v0, v1);
     }
 }
-static_assert(kTimeFeat % 2 == 0 && kLogTimeFeat % 2 == 0 && kFourierFeat % 2 == 0, "features come in pairs");
-
 // A warp takes 32 rows, their dot products one after the other (the row's 1 KB
 // coalesced, the next row's loads in flight), then each lane turns one row's
 // outputs into G: the FP64 exponential and sine-cosine run on 32 lanes instead
@@ -1209,7 +1348,8 @@ void launch_mode(cudaStream_t s, const CUtensorMap& ta, const CUtensorMap& tb, d
 int prepare_gemm() {
     static std::atomic<bool> done{false};
     if (!done.load(std::memory_order_relaxed) && set_attr<kFwdTrain>() && set_attr<kBwdData>() && set_attr<kWgrad>() &&
-        cudaFuncSetAttribute(k_layer_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kInfSmem) == cudaSuccess)
+        cudaFuncSetAttribute(k_layer_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kInfSmem) == cudaSuccess &&
+        cudaFuncSetAttribute(k_head_train, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(HeadShared)) == cudaSuccess)
         done.store(true, std::memory_order_relaxed);
     return done.load(std::memory_order_relaxed) ? 0 : 3;
 }
@@ -1251,12 +1391,13 @@ int launch_gemm(cudaStream_t s, int mode, const bf16* A, const bf16* B, int rows
 void launch_step_begin(cudaStream_t s, TrainScalars* ts) { launch_dep(k_step_begin, dim3(1), dim3(1), 0, s, ts); }
 
 void launch_batch(cudaStream_t s, const BatchArgs& a) {
-    launch_dep(k_batch, dim3(a.B / kBatchRows), dim3(kIn), 0, s, a);
+    launch_dep(k_batch, dim3(a.B / kBatchRows), dim3(kBatchThreads), 0, s, a);
 }
 
 void launch_head_train(cudaStream_t s, const bf16* H, const bf16* Z, const float* W6, const float* b6, const float* Y,
                        const float* C, int B, bf16* dZ, bf16* dZT, float* gpart, float* lpart) {
-    launch_dep(k_head_train, dim3(B / kHeadRows), dim3(256), 0, s, H, Z, W6, b6, Y, C, B, dZ, dZT, gpart, lpart);
+    launch_dep(k_head_train, dim3(B / kHeadRows), dim3(256), sizeof(HeadShared), s,  // prepare_gemm set the limit
+               H, Z, W6, b6, Y, C, B, dZ, dZT, gpart, lpart);
 }
 
 void launch_bias_grad(cudaStream_t s, const bf16* const* dZT, int layers, int B, float* gb) {
@@ -1283,8 +1424,12 @@ void launch_transposes(cudaStream_t s, const AdamArgs& a) {
 }  // namespace
 
 void launch_adam(cudaStream_t s, const AdamArgs& a, long long) {
-    launch_dep(k_adam, dim3((unsigned)((max_seg(a) + 255) / 256), a.nseg), dim3(256), 0, s, a);
-    launch_transposes(s, a);
+    long long blocks = 1;
+    for (int q = 0; q < a.nseg; q++) {
+        const long long per = adam_items(a.seg[q]);
+        blocks = std::max(blocks, (a.seg[q].n + per - 1) / per);
+    }
+    launch_dep(k_adam, dim3((unsigned)blocks, a.nseg), dim3(256), 0, s, a);
 }
 
 void launch_sync_weights(cudaStream_t s, const AdamArgs& a, long long) {

@@ -136,8 +136,8 @@ struct AdamArgs {
     float eps, weight_decay;
     const TrainScalars* ts;
 };
-// AdamW over every segment (one grid row per segment), then the BF16
-// transposes W^T of the weight segments (32 x 32 shared-memory tiles).
+// AdamW over every segment (one grid row per segment); refreshes W and W^T of
+// the weight segments, whose rows and columns are multiples of 32.
 void launch_adam(cudaStream_t s, const AdamArgs& a, long long nparam);
 // bf16 copies of every weight segment from the master parameters.
 void launch_sync_weights(cudaStream_t s, const AdamArgs& a, long long nparam);

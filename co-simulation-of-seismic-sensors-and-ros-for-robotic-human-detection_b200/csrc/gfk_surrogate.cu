@@ -256,8 +256,9 @@ int enqueue_fwd_bwd(gfk_net* n, bool train_step) {
     M::launch_bias_grad(s, dzt, kLayers, B, n->gb);
     n->ctx->launches++;
     if (train_step) {
+        M::launch_step_begin(s, n->d_ts);
         M::launch_loss_hist(s, n->lpart, n->B / M::kHeadRows, n->B, n->d_ts, n->hist, kHistCap);
-        n->ctx->launches++;
+        n->ctx->launches += 2;
     }
     SG_CUDA(n->ctx, cudaEventRecord(n->ev_join, n->side));
     SG_CUDA(n->ctx, cudaStreamWaitEvent(s, n->ev_join, 0));
@@ -266,7 +267,6 @@ int enqueue_fwd_bwd(gfk_net* n, bool train_step) {
 
 int enqueue_step(gfk_net* n, const gfk_dataset* d) {
     cudaStream_t s = n->ctx->stream;
-    M::launch_step_begin(s, n->d_ts);
     M::BatchArgs b{};
     b.labels = d->d_labels;
     b.lmax = d->d_lmax;
@@ -297,10 +297,10 @@ int enqueue_step(gfk_net* n, const gfk_dataset* d) {
     b.Y = n->Y;
     b.C = n->Cw;
     M::launch_batch(s, b);
-    n->ctx->launches += 2;
+    n->ctx->launches++;
     SG_TRY(enqueue_fwd_bwd(n, true));
     M::launch_adam(s, n->adam, n->nparam);
-    n->ctx->launches += 2;
+    n->ctx->launches++;
     return GFK_OK;
 }
 
