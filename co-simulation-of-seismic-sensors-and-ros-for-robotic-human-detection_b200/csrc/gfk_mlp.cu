@@ -16,7 +16,8 @@
 // writes W and W^T. The kernel shape is the wavenumber-sum kernel's: one
 // 128 x 128 tile per CTA, warp 0 TMA, warp 1 TMEM + MMA issue, warps 2-5
 // epilogue, SWIZZLE_64B tiles (32 BF16 = 64 bytes per row), 3-stage ring,
-// bounded waits. Inference has a kernel of its own, k_layer_infer. No load is multicast.
+// bounded waits. Inference on many rows has a kernel of its own,
+// k_layer_infer. No load is multicast.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <math_constants.h>
@@ -200,7 +201,7 @@ __global__ void __launch_bounds__(THREADS, 2)
         // BF16 results go to a shared-memory tile (the pipeline stages are free
         // once every MMA has completed), FP32 gradient partials straight out
         // the tile's bias columns, read once while the MMAs run
-        if (MODE == kFwdTrain) {
+        if (MODE == kFwdTrain || MODE == kFwdInfer) {
             bias_s[threadIdx.x - 64] = a.bias[n0 + threadIdx.x - 64];
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
@@ -242,14 +243,14 @@ __global__ void __launch_bounds__(THREADS, 2)
                 continue;
             }
             float y[32];
-            if (MODE == kFwdTrain) {
+            if (MODE == kFwdTrain || MODE == kFwdInfer) {
                 float zv[32];
 #pragma unroll
                 for (int c = 0; c < 32; c++) {
                     zv[c] = __uint_as_float(v[c]) + bias_s[j * 32 + c];
                     y[c] = zv[c] * sigmoid_(zv[c]);
                 }
-                {
+                if (MODE == kFwdTrain) {
                     uint4* zd = reinterpret_cast<uint4*>(tileZ + rl * kTileLd + j * 32);
 #pragma unroll
                     for (int c = 0; c < 4; c++)
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(THREADS, 2)
             if (MODE == kFwdTrain)
                 *reinterpret_cast<uint4*>(a.zout + g) = *reinterpret_cast<const uint4*>(tileZ + r * kTileLd + c8);
         }
-        if (a.outT) {
+        if (MODE != kFwdInfer && a.outT) {
             // 32 bytes (16 rows) of one transposed row per thread; lanes run
             // over columns, so the shared-memory column reads do not conflict
             for (int c = threadIdx.x; c < BN * (BM / 16); c += THREADS) {
@@ -356,7 +357,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kInfThreads, 1)
     uint8_t* outs = ring + kInfStages * kInfBlock;  // one box per group
     float* bias_s = reinterpret_cast<float*>(outs + kInfGroups * kInfBox);
     uint64_t* w_full = reinterpret_cast<uint64_t*>(bias_s + kInfN);
-    uint64_t* a_full = w_full + 1;
+    uint64_t* a_full = w_full + kInfKb;
     uint64_t* a_empty = a_full + kInfStages;
     uint64_t* acc_full = a_empty + kInfStages;
     uint64_t* acc_empty = acc_full + 2;
@@ -371,7 +372,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kInfThreads, 1)
     const int n0 = ((blockIdx.x >> 1) % nslab) * kInfN;                             // the pair's columns
     const int mb0 = (blockIdx.x >> 1) / nslab, mstep = (gridDim.x >> 1) / nslab;    // and row blocks
     if (threadIdx.x == 0) {
-        mbar_init(w_full, 1);
+        for (int i = 0; i < kInfKb; i++) mbar_init(&w_full[i], 1);
         for (int i = 0; i < kInfStages; i++) {
             mbar_init(&a_full[i], 1);
             mbar_init(&a_empty[i], 1);
@@ -403,10 +404,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kInfThreads, 1)
     if (warp == 0) {
         if (lane == 0) {
             const int row0 = rank * BM;
-            if (rank == 0) mbar_expect_tx(w_full, 2 * nkb * kInfBlock);
-            const uint32_t wbar = leader_addr(w_full);
-            for (int kb = 0; kb < nkb; kb++)
-                tma_load_2d_pair(smem + kb * kInfBlock, &tmB, wbar, kb * BK, n0 + row0);
             int st = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -415,6 +412,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kInfThreads, 1)
                     if (!mbar_wait(&a_empty[st], ph ^ 1)) {
                         ok = false;
                         break;
+                    }
+                    if (mb == mb0) {  // the weights come with the first block: its MMAs start on the first K block
+                        if (rank == 0) mbar_expect_tx(&w_full[kb], 2 * kInfBlock);
+                        tma_load_2d_pair(smem + kb * kInfBlock, &tmB, leader_addr(&w_full[kb]), kb * BK, n0 + row0);
                     }
                     if (rank == 0) mbar_expect_tx(&a_full[st], 2 * kInfBlock);
                     tma_load_2d_pair(ring + st * kInfBlock, &tmA, leader_addr(&a_full[st]), kb * BK, mb * 2 * BM + row0);
@@ -430,7 +431,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kInfThreads, 1)
             const uint32_t idesc = idesc_bf16(2 * BM, kInfN);
             int st = 0, tile = 0;
             uint32_t ph = 0;
-            bool ok = leader_wait(w_full, 0);
+            bool ok = true;
             for (int mb = mb0; mb < nblock && ok; mb += mstep, tile++) {
                 const int buf = tile & 1;
                 if (!leader_wait(&acc_empty[buf], ((tile >> 1) & 1) ^ 1) || *abort_flag) {
@@ -438,7 +439,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kInfThreads, 1)
                     break;
                 }
                 for (int kb = 0; kb < nkb; kb++) {
-                    if (!leader_wait(&a_full[st], ph) || *abort_flag) {
+                    if ((mb == mb0 && !leader_wait(&w_full[kb], 0)) || !leader_wait(&a_full[st], ph) || *abort_flag) {
                         ok = false;
                         break;
                     }
@@ -1347,7 +1348,7 @@ void launch_mode(cudaStream_t s, const CUtensorMap& ta, const CUtensorMap& tb, d
 
 int prepare_gemm() {
     static std::atomic<bool> done{false};
-    if (!done.load(std::memory_order_relaxed) && set_attr<kFwdTrain>() && set_attr<kBwdData>() && set_attr<kWgrad>() &&
+    if (!done.load(std::memory_order_relaxed) && set_attr<kFwdTrain>() && set_attr<kFwdInfer>() && set_attr<kBwdData>() && set_attr<kWgrad>() &&
         cudaFuncSetAttribute(k_layer_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kInfSmem) == cudaSuccess &&
         cudaFuncSetAttribute(k_head_train, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(HeadShared)) == cudaSuccess)
         done.store(true, std::memory_order_relaxed);
@@ -1373,6 +1374,15 @@ int launch_gemm(cudaStream_t s, int mode, const bf16* A, const bf16* B, int rows
             if (cudaGetDevice(&dev) != cudaSuccess ||
                 cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
                 return 3;
+            // While every tile has a place of its own (two CTAs per SM) k_gemm is
+            // ahead: its CTAs start beside the previous layer's, those with all of an
+            // SM's shared memory cannot. A prediction of 1 / 2048 / 8192 rows: 132 / 175 /
+            // 236 us, with the pairs 158 / 200 / 248; of 12288 / 16384 / 2^20: 297 / 319 /
+            // 5530 against 303 / 319 / 3750.
+            if (rowsA / BM * (rowsB / BN) <= 2 * sms) {
+                launch_mode<kFwdInfer>(s, ta, tb, grid, a);
+                return 0;
+            }
             CUtensorMap to;
             if (!make_map_bf16(&ta, A, rowsA, ktotal, true) || !make_map_bf16(&tb, B, rowsB, ktotal, true) ||
                 !make_map_bf16(&to, a.out, rowsA, rowsB, true))

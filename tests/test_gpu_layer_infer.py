@@ -7,7 +7,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# 37 blocks (one each), 38 (a second for one pair), 111 and a ragged last 128 rows, 236
+# 9472 rows, the last count with a tile per CTA, then pairs: a second block for one pair, a
+# last block of 128 rows, 236 blocks; each against 256 to 1024 rows, a tile per CTA
 @pytest.mark.parametrize("ns,nf,nr", [(37, 256, 1), (37, 257, 1), (37, 769, 1), (59, 512, 2)])
 def test_rows_do_not_depend_on_their_block(gfk, engine, ns, nf, nr):
     net = gfk.surrogate.Net(gfk.surrogate.NetConfig(batch=128, seed=12), engine)
