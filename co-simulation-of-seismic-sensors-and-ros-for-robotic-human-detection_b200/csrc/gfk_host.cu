@@ -192,6 +192,17 @@ struct TimedSeg {
     bool pending;
 };
 
+// (row, wavenumber) points up to which a plan solves every one instead of panels'
+// nodes: about ten solves per resident thread (148 SMs x 640). A panel that is refused
+// goes through three solves one after the other and its neighbours in the item wait,
+// which only pays once there are many items. Execute of a plan, every point / panels:
+//   629 x 16 rows, 9 layers 69 / 85 us       2428 x 120, 11 layers 123 / 159 us
+//   2408 x 165, 8 layers 121 / 148 us        1384 x 670, 6 layers 161 / 162 us
+//   8819 x 109, 3 layers 127 / 114 us        9695 x 116, 9 layers 222 / 205 us
+//   8419 x 264, 5 layers 259 / 209 us        15439 x 324, 9 layers 734 / 452 us
+// The plan's total decides, so its chunks agree, and a forced shape has panels.
+constexpr int64_t kDirectPoints = 950000;
+
 struct gfk_plan {
     gfk_ctx* ctx = nullptr;
     gfk_solve solve{};
@@ -240,6 +251,7 @@ struct gfk_plan {
     int32_t launches_per_exec = 0;  // after the first execute (which may also build the Hankel weights)
     std::shared_ptr<gfk_weights> wts;  // d_W or d_B, shared with other plans on the same grid and ranges
     int prop_variant = -1;       // Dunkin launch shape; -1 until the first execute tunes it
+    bool direct = false;         // every wavenumber solved, no panels (kDirectPoints)
     std::vector<float> tune_ms;  // per variant, from the tuning run
     int tc_variant = -1;            // tensor-core sum tile shape; -1 until the first execute tunes it
     std::vector<float> tc_tune_ms;  // per shape, from the tuning run
@@ -717,7 +729,9 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         if (p->chunk_begin[c + 1] > p->chunk_begin[c]) nchunks++;
     p->launches_per_exec = p->nf > 0 ? (p->shared ? 2 : 1) + 2 * nchunks : 0;
     if (p->nf > 0 && (p->ksplit > 1 || !p->shared)) p->launches_per_exec += nchunks;
-    if (p->fused || !p->shared) p->prop_variant = 0;  // one launch shape; nothing to tune
+    p->direct = p->solve.formulation == GFK_DUNKIN && p->shared && !p->fused &&
+                (int64_t)p->nf * p->max_nk <= kDirectPoints && !getenv("GFK_PROP_VARIANT");
+    if (p->fused || !p->shared || p->direct) p->prop_variant = 0;  // one launch shape; nothing to tune
     *out = p;
     return GFK_OK;
 }
@@ -932,7 +946,8 @@ int plan_enqueue(gfk_plan* p, bool timed) {
             GFK_CUDA(ctx, cudaMemsetAsync(p->d_queue, 0, sizeof(unsigned int), s));
         if (timed && (st = begin_seg(p, 0, &seg))) return st;
         gfk::launch_prop(s, p->d_lc, p->d_media, p->d_fd + fb, p->d_wc2 + fb, cnf, cmax, p->d_C + fb, form, ctx->panels, p->d_rem,
-                         p->d_status + fb, std::max(p->prop_variant, 0), p->tc ? &so : nullptr, p->d_queue);
+                         p->d_status + fb, p->direct ? gfk::kPropDirect : std::max(p->prop_variant, 0),
+                         p->tc ? &so : nullptr, p->d_queue);
         if (timed && (st = end_seg(p, seg))) return st;
         if (timed && (st = begin_seg(p, 1, &seg))) return st;
         if (p->tc) {

@@ -155,8 +155,9 @@ void launch_static(cudaStream_t s, const LayerC* lc, const MediumP* media, const
 // persistent: each resident block takes items from a device queue, last row
 // first, until none are left. The row's layer constants are staged in shared memory.
 // Launch shapes are template parameters; the plan times them once and keeps
-// the fastest. The direct formulation solves every wavenumber: its parity with
-// the reference includes the digits its eigenbasis loses.
+// the fastest. The direct formulation (FORM 0) solves every wavenumber: its parity with
+// the reference includes the digits its eigenbasis loses. So does FORM 2, the Dunkin
+// solve of small banks (kDirectPoints), a wavenumber per thread.
 
 constexpr int kNodeStride = kPanelN + 4;  // of the node values in shared memory: conflict-free B fragments
 
@@ -407,14 +408,19 @@ __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const M
     cd* row = rem + fdesc.off;
     int bad = 0;
     double mre = 0.0, mim = 0.0;
-    if constexpr (FORM == 0) {
+    if constexpr (FORM != 1) {
         const int i = run * THREADS + threadIdx.x + 1;
         if (i <= n) {
-            bool ok;
             const double k = (double)i * d;
-            cd u = direct_u(sm.lc, nl, kTwoPi * fdesc.freq, k, mu_ref, ok);
-            if (!ok) bad |= kStSingular;
-            cd r = k * u - c;
+            cd r;
+            if constexpr (FORM == 0) {
+                bool ok;
+                cd u = direct_u(sm.lc, nl, kTwoPi * fdesc.freq, k, mu_ref, ok);
+                if (!ok) bad |= kStSingular;
+                r = k * u - c;
+            } else {
+                r = k * dunkin_u(sm.lc, nl, wc2[f], k, mu_ref) - c;
+            }
             if (!finite_cd(r)) { bad |= kStNonfinite; r = mk(0.0); }
             row[i - 1] = r;
             mre = fabs(r.re);
@@ -644,6 +650,14 @@ void launch_prop(cudaStream_t s, const LayerC* lc, const MediumP* media, const F
             k_prop<0, 128, 1, false, true><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
         else
             k_prop<0, 128, 1, false, false><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
+        return;
+    }
+    if (variant == kPropDirect) {
+        const dim3 grid((max_nk + 127) / 128, nf);
+        if (slice)
+            k_prop<2, 128, 5, false, true><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
+        else
+            k_prop<2, 128, 5, false, false><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
         return;
     }
     if (variant < 0 || variant >= kPropVariants) variant = 0;

@@ -52,6 +52,7 @@ int rows_item_size(long long wavenumbers, int nr);
 void launch_prop(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, const cd* wc2, int nf,
                  int max_nk, const cd* C, int formulation, const double* tab, cd* rem, int* status, int variant = 0,
                  const SliceOut* slice = nullptr, unsigned int* queue = nullptr);
+constexpr int kPropDirect = -1;  // `variant` of the Dunkin launch that solves every wavenumber
 int prop_variant_count();
 bool prop_variant_persistent(int variant);
 // threads per block, blocks per SM it is compiled for, wavenumbers per thread
