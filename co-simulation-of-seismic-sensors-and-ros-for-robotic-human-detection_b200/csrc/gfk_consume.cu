@@ -161,7 +161,14 @@ void launch_impulse(cudaStream_t s, const ImpulseArgs& a, int nq) {
     const int m = a.n / 2;
     const int smem = fft_room(m) * (int)sizeof(cd);  // at most 36.9 KB: no opt-in
     static_assert(fft_room(kMaxSamples / 2) * sizeof(cd) <= 48 * 1024, "shared memory");
-    k_impulse<<<nq, m >= 256 ? m / 8 : 32, smem, s>>>(a);
+    // The transform takes m / 8 threads. While every block is resident at once (4 of
+    // kThreads on each of 148 SMs) the spectrum takes a thread per pair of bins, up to
+    // kThreads: 16 / 592 queries of 1024 points 34.7 / 38.4 -> 29.2 / 33.7 us, of
+    // 2048 35.8 / 43.6 -> 32.4 / 41.1; of more the idle threads cost: 2368 of 1024 54.3 -> 58.3.
+    constexpr int kResident = 4 * 148;
+    int threads = m >= 256 ? m / 8 : 32;
+    if (nq <= kResident) threads = std::max(threads, std::min(kThreads, (m / 2 + 32) / 32 * 32));
+    k_impulse<<<nq, threads, smem, s>>>(a);
 }
 
 }  // namespace consume

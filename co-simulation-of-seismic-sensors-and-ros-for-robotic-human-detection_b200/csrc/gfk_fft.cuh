@@ -71,8 +71,8 @@ __device__ __forceinline__ void dft_small(cd (&v)[R]) {
 __device__ __forceinline__ int fft_at(int i) { return i + (i >> 3); }
 __host__ __device__ constexpr int fft_room(int m) { return m + m / 8 + 1; }
 
-// One radix-R Stockham pass over m values by max(32, m / 8) threads, each with
-// up to 8 / R butterflies: loads x, then (all threads) emit(element, value)
+// One radix-R Stockham pass over m values by the block's first max(32, m / 8)
+// threads, each with up to 8 / R butterflies: loads x, then (all threads) emit(element, value)
 // for every output. tw[q] = e^{-2 pi i q / tn}, q < tn/2, tn a multiple of m;
 // ns is the product of the radices before. Twiddles: w, w^2, w^4 from the
 // table, the others as their products.
@@ -84,7 +84,7 @@ __device__ __forceinline__ void fft_pass(const cd* x, int m, int ns, const cd* _
 #pragma unroll
     for (int b = 0; b < B; b++) {
         const int j = tid + b * nt;
-        if (j < stride) {
+        if (tid < nt && j < stride) {
 #pragma unroll
             for (int r = 0; r < R; r++) v[b][r] = x[fft_at(j + r * stride)];
         }
@@ -93,7 +93,7 @@ __device__ __forceinline__ void fft_pass(const cd* x, int m, int ns, const cd* _
 #pragma unroll
     for (int b = 0; b < B; b++) {
         const int j = tid + b * nt;
-        if (j >= stride) continue;
+        if (tid >= nt || j >= stride) continue;
         const int k = j & (ns - 1);
         if (ns > 1) {
             const int q = k * (tn / (ns * R));
@@ -122,7 +122,7 @@ __device__ __forceinline__ void fft_pass(const cd* x, int m, int ns, const cd* _
 
 // Forward transform (e^{-i}) of the m = 2^logm values at x[fft_at(i)], the last
 // pass handing its outputs, in natural order, to emit(i, value) instead of
-// shared memory. The block has max(32, m / 8) threads; all must call it, with
+// shared memory. The block has at least max(32, m / 8) threads; all must call it, with
 // x written and a barrier passed. Every pass but the first is radix 8: a third of the
 // passes (and of the shared-memory traffic and barriers) of radix 2.
 template <class Emit>
