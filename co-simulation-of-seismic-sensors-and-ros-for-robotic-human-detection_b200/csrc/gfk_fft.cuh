@@ -84,7 +84,7 @@ __device__ __forceinline__ void fft_pass(const cd* x, int m, int ns, const cd* _
 #pragma unroll
     for (int b = 0; b < B; b++) {
         const int j = tid + b * nt;
-        if (tid < nt && j < stride) {
+        if ((B == 1 || tid < nt) && j < stride) {
 #pragma unroll
             for (int r = 0; r < R; r++) v[b][r] = x[fft_at(j + r * stride)];
         }
@@ -93,7 +93,7 @@ __device__ __forceinline__ void fft_pass(const cd* x, int m, int ns, const cd* _
 #pragma unroll
     for (int b = 0; b < B; b++) {
         const int j = tid + b * nt;
-        if (tid >= nt || j >= stride) continue;
+        if ((B > 1 && tid >= nt) || j >= stride) continue;
         const int k = j & (ns - 1);
         if (ns > 1) {
             const int q = k * (tn / (ns * R));
