@@ -787,7 +787,7 @@ int gfk_net_train_ranges(gfk_net* n, gfk_dataset* d, const int32_t* train, int32
         n->graph_train.assign(train, train + ntrain);
     }
     // launches per replayed step, counted from the step's own enqueue
-    const int64_t per_step = 2 + kLayers + 1 + (kLayers - 1) + kLayers + 1 + 3;
+    const int64_t per_step = 2 + kLayers + 1 + (kLayers - 1) + kLayers + 1 + 2;
     std::vector<float> h(kHistCap * 2);
     for (int done = 0; done < steps;) {
         const int blk = std::min(kHistCap, steps - done);
