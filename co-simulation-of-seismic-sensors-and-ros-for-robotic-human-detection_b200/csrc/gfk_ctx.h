@@ -58,7 +58,7 @@ struct gfk_ctx {
     // page-locked memory that small results come back through, one call at a time
     static constexpr size_t kBounce = size_t(1) << 20;
     void* bounce = nullptr;
-    double* panels = nullptr;  // the panel interpolation table (gfk_panel.cuh), built by gfk_open
+    double* panels = nullptr;  // the panel interpolation table (gfk_panel.cuh), from the first Dunkin plan on
     // the most recent plan's Hankel weights, kept for the next plan
     std::shared_ptr<gfk_weights> weights;
 };
