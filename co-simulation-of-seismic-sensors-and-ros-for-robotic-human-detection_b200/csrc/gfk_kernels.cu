@@ -285,7 +285,7 @@ __device__ __forceinline__ void panel_item(const double* __restrict__ tab, SMEM&
             double mid;
             const double tail = panel_tail<1, true>(tab + kPtRowsE, v, mid);
             const double scale = cabs1 + big;
-            mode = use && tail <= kPanelTol * scale;
+            mode = use && panel_passes(tail, scale);
             // decay per 6 orders, q = tail/mid; at order 31: tail q^(16/6) <= 10 tol scale
             const float s = (float)(1.0 / scale), tl = (float)tail * s, q = tl / ((float)mid * s);
             const float room = (float)(10.0 * kPanelTol) / tl, q2 = q * q, q4 = q2 * q2;
@@ -297,7 +297,7 @@ __device__ __forceinline__ void panel_item(const double* __restrict__ tab, SMEM&
                 const cd v[2] = {first, r};
                 double none;
                 const double tail = panel_tail<2, false>(tab + kPtRowsN, v, none);
-                if (more && tail <= kPanelTol * (cabs1 + fmax(big, m2))) mode = 2;
+                if (more && panel_passes(tail, cabs1 + fmax(big, m2))) mode = 2;
             }
             if constexpr (NR > 0) {
                 if (mode) {

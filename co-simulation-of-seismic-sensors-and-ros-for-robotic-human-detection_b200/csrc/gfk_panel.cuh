@@ -24,6 +24,8 @@
 // another 5-12%. Panels of 256 with 32/16 nodes were within 12% of these; 64/32
 // nodes save less.
 #pragma once
+#include <cmath>
+#include <utility>
 #include <vector>
 
 #include "gfk_math.cuh"
@@ -35,6 +37,12 @@ constexpr int kPanelE = 16;        // nodes of the first try
 constexpr int kPanelN = 32;        // nodes of both
 constexpr int kPanelLeast = 33;    // a shorter last panel is solved directly: no more solves than its second try
 constexpr double kPanelTol = 1e-15;  // last coefficients against |C| + max |k u - C|
+
+// Whether a panel may be interpolated: `tail` its largest last coefficient (infinite
+// where one is not finite), `scale` |C| + max |k u - C| over its nodes. A node that
+// overflowed makes both infinite, and Inf <= tol Inf holds, so the scale has to be finite:
+// a refused panel's wavenumbers are solved one by one and flagged there.
+GFK_HD bool panel_passes(double tail, double scale) { return scale < INFINITY && tail <= kPanelTol * scale; }
 
 // Offsets (doubles) into the table every context keeps on the device.
 constexpr int kPtX = 0;                              // node abscissae, first 16 then the other 16
