@@ -192,16 +192,22 @@ struct TimedSeg {
     bool pending;
 };
 
-// (row, wavenumber) points up to which a plan solves every one instead of panels'
-// nodes: about ten solves per resident thread (148 SMs x 640). A panel that is refused
-// goes through three solves one after the other and its neighbours in the item wait,
-// which only pays once there are many items. Execute of a plan, every point / panels:
-//   629 x 16 rows, 9 layers 69 / 85 us       2428 x 120, 11 layers 123 / 159 us
-//   2408 x 165, 8 layers 121 / 148 us        1384 x 670, 6 layers 161 / 162 us
-//   8819 x 109, 3 layers 127 / 114 us        9695 x 116, 9 layers 222 / 205 us
-//   8419 x 264, 5 layers 259 / 209 us        15439 x 324, 9 layers 734 / 452 us
+// Whether a plan's rows have every wavenumber solved instead of panels' nodes:
+// short rows always, others up to about ten solves per resident thread (148 SMs x 640).
+// A panel that is refused goes through three solves one after the other and its
+// neighbours in the item (8 panels) wait, which only pays once there are many items,
+// and full ones; a row's coarse grid is also refused more often. Execute of a plan,
+// every point / panels:
+//   5062 rows x 251, 12 layers 347 / 489 us   2673 x 691, 6 layers 255 / 318 us
+//   1735 x 939, 12 layers 363 / 385 us        1295 x 1044, 6 layers 204 / 200 us
+//   120 x 2428, 11 layers 123 / 159 us        670 x 1384, 6 layers 161 / 162 us
+//   109 x 8819, 3 layers 127 / 114 us         116 x 9695, 9 layers 222 / 205 us
+//   264 x 8419, 5 layers 259 / 209 us         324 x 15439, 9 layers 734 / 452 us
 // The plan's total decides, so its chunks agree, and a forced shape has panels.
 constexpr int64_t kDirectPoints = 950000;
+bool solves_every_point(int64_t rows, int nk) {
+    return (nk <= 128 * gfk::kRowSweeps || rows * nk <= kDirectPoints) && !getenv("GFK_PROP_VARIANT");
+}
 
 struct gfk_plan {
     gfk_ctx* ctx = nullptr;
@@ -251,7 +257,7 @@ struct gfk_plan {
     int32_t launches_per_exec = 0;  // after the first execute (which may also build the Hankel weights)
     std::shared_ptr<gfk_weights> wts;  // d_W or d_B, shared with other plans on the same grid and ranges
     int prop_variant = -1;       // Dunkin launch shape; -1 until the first execute tunes it
-    bool direct = false;         // every wavenumber solved, no panels (kDirectPoints)
+    bool direct = false;         // every wavenumber solved, no panels (solves_every_point)
     std::vector<float> tune_ms;  // per variant, from the tuning run
     int tc_variant = -1;            // tensor-core sum tile shape; -1 until the first execute tunes it
     std::vector<float> tc_tune_ms;  // per shape, from the tuning run
@@ -623,6 +629,7 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         p->fused = true;
         p->tc = false;
     }
+    p->direct = p->shared && !p->fused && s->formulation == GFK_DUNKIN && solves_every_point(p->nf, p->g_n);
     // row chunks bounded by the integrand budget and the grid limit; on a shared
     // grid every row keeps its dense slot (row x Nk), failed rows included
     const int64_t budget = kDefaultRemBudget / (int64_t)sizeof(cd);
@@ -736,7 +743,7 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         p->ksplit = ks;
         if (ks > 1) lay.add(&p->d_ksum, (size_t)(ks * per_split));
     }
-    if (!st && p->solve.formulation == GFK_DUNKIN) st = ensure_panels(ctx);
+    if (!st && p->solve.formulation == GFK_DUNKIN && !p->direct) st = ensure_panels(ctx);
     if (!st) st = lay.make(ctx, p->owned);
     if (st) {
         plan_free(p);
@@ -748,9 +755,13 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         if (p->chunk_begin[c + 1] > p->chunk_begin[c]) nchunks++;
     p->launches_per_exec = p->nf > 0 ? (p->shared ? 2 : 1) + 2 * nchunks : 0;
     if (p->nf > 0 && (p->ksplit > 1 || !p->shared)) p->launches_per_exec += nchunks;
-    p->direct = p->solve.formulation == GFK_DUNKIN && p->shared && !p->fused &&
-                (int64_t)p->nf * p->max_nk <= kDirectPoints && !getenv("GFK_PROP_VARIANT");
-    if (p->fused || !p->shared || p->direct) p->prop_variant = 0;  // one launch shape; nothing to tune
+    // plans of one launch shape, nothing to tune
+    if (p->direct)
+        p->prop_variant = gfk::direct_variant(p->max_nl, p->nf, p->g_n);
+    else if (!p->shared && p->solve.formulation == GFK_DUNKIN)
+        p->prop_variant = gfk::kPropRows;
+    else if (p->fused || !p->shared)
+        p->prop_variant = 0;
     *out = p;
     return GFK_OK;
 }
@@ -965,7 +976,7 @@ int plan_enqueue(gfk_plan* p, bool timed) {
             GFK_CUDA(ctx, cudaMemsetAsync(p->d_queue, 0, sizeof(unsigned int), s));
         if (timed && (st = begin_seg(p, 0, &seg))) return st;
         gfk::launch_prop(s, p->d_lc, p->d_media, p->d_fd + fb, p->d_wc2 + fb, cnf, cmax, p->d_C + fb, form, ctx->panels, p->d_rem,
-                         p->d_status + fb, p->direct ? gfk::kPropDirect : std::max(p->prop_variant, 0),
+                         p->d_status + fb, std::max(p->prop_variant, 0),
                          p->tc ? &so : nullptr, p->d_queue);
         if (timed && (st = end_seg(p, seg))) return st;
         if (timed && (st = begin_seg(p, 1, &seg))) return st;

@@ -157,7 +157,8 @@ void launch_static(cudaStream_t s, const LayerC* lc, const MediumP* media, const
 // Launch shapes are template parameters; the plan times them once and keeps
 // the fastest. The direct formulation (FORM 0) solves every wavenumber: its parity with
 // the reference includes the digits its eigenbasis loses. So does FORM 2, the Dunkin
-// solve of small banks (kDirectPoints), a wavenumber per thread.
+// solve of short rows and small banks (direct_variant), SWEEPS runs of 128
+// wavenumbers a block, a wavenumber per thread in each.
 
 constexpr int kNodeStride = kPanelN + 4;  // of the node values in shared memory: conflict-free B fragments
 
@@ -388,7 +389,7 @@ __device__ __forceinline__ void panel_item(const double* __restrict__ tab, SMEM&
 }
 
 // `stage`: the block's staged layer constants are not row f's (uniform).
-template <int FORM, int THREADS, bool WIDE, bool SLICE>
+template <int FORM, int THREADS, bool WIDE, bool SLICE, int SWEEPS = 1>
 __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const MediumP* __restrict__ media,
                                           const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2,
                                           const cd* __restrict__ C, const double* __restrict__ tab,
@@ -409,8 +410,10 @@ __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const M
     int bad = 0;
     double mre = 0.0, mim = 0.0;
     if constexpr (FORM != 1) {
-        const int i = run * THREADS + threadIdx.x + 1;
-        if (i <= n) {
+#pragma unroll 1
+        for (int sweep = 0; sweep < SWEEPS; sweep++) {
+            const int i = (run * SWEEPS + sweep) * THREADS + threadIdx.x + 1;
+            if (i > n) break;
             const double k = (double)i * d;
             cd r;
             if constexpr (FORM == 0) {
@@ -423,8 +426,8 @@ __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const M
             }
             if (!finite_cd(r)) { bad |= kStNonfinite; r = mk(0.0); }
             row[i - 1] = r;
-            mre = fabs(r.re);
-            mim = fabs(r.im);
+            mre = fmax(mre, fabs(r.re));
+            mim = fmax(mim, fabs(r.im));
         }
     } else {
         panel_item<THREADS, WIDE, 0, true>(tab, sm, nl, mu_ref, wc2[f], c, d, n, run * THREADS * (WIDE ? 4 : 8), n, row,
@@ -471,7 +474,7 @@ __device__ __forceinline__ void prop_item(const LayerC* __restrict__ lc, const M
     }
 }
 
-template <int FORM, int THREADS, int MINB, bool WIDE, bool SLICE>
+template <int FORM, int THREADS, int MINB, bool WIDE, bool SLICE, int SWEEPS = 1>
 __global__ __launch_bounds__(THREADS, MINB) void k_prop(const LayerC* __restrict__ lc,
                                                        const MediumP* __restrict__ media,
                                                        const FreqDesc* __restrict__ fd, const cd* __restrict__ wc2,
@@ -479,8 +482,8 @@ __global__ __launch_bounds__(THREADS, MINB) void k_prop(const LayerC* __restrict
                                                        cd* __restrict__ rem, int* __restrict__ status, SliceOut so,
                                                        PropQueue) {
     __shared__ PropSmem<THREADS, SLICE> sm;
-    prop_item<FORM, THREADS, WIDE, SLICE>(lc, media, fd, wc2, C, tab, rem, status, so, gridDim.y - 1 - blockIdx.y, blockIdx.x,
-                                    gridDim.x, true, sm);
+    prop_item<FORM, THREADS, WIDE, SLICE, SWEEPS>(lc, media, fd, wc2, C, tab, rem, status, so,
+                                                  gridDim.y - 1 - blockIdx.y, blockIdx.x, gridDim.x, true, sm);
 }
 
 // Rows of uneven length: block (item, y) serves the y-th run of 128
@@ -599,6 +602,20 @@ const PropVariant kDunkinVariants[] = {
     GFK_PROP_QUEUE(128, 5, true),
 };
 constexpr int kPropVariants = sizeof(kDunkinVariants) / sizeof(kDunkinVariants[0]);
+
+// The launches that solve every wavenumber (FORM 2), variants kPropFixed + index.
+struct DirectVariant {
+    PropFn fn, fn_slice;
+    int threads, minb, sweeps;
+};
+#define GFK_DIRECT(B, S) {k_prop<2, 128, B, false, false, S>, k_prop<2, 128, B, false, true, S>, 128, B, S}
+const DirectVariant kDirectVariants[] = {
+    GFK_DIRECT(4, 1),           // <= 128 registers
+    GFK_DIRECT(5, 1),           // <= 96 registers
+    GFK_DIRECT(5, kRowSweeps),  // a short row per block
+};
+constexpr int kDirectCount = sizeof(kDirectVariants) / sizeof(kDirectVariants[0]);
+#undef GFK_DIRECT
 #undef GFK_PROP_SHAPE
 #undef GFK_PROP_QUEUE
 
@@ -628,7 +645,33 @@ bool prop_variant_persistent(int variant) {
     return variant >= 0 && variant < kPropVariants && kDunkinVariants[variant].persistent;
 }
 
+// Which of kDirectVariants a plan of `rows` rows of nk wavenumbers takes. Plan execute on
+// either side of each line (us; first the fastest of the 13 shapes that used to be timed
+// for each plan, then these three in turn):
+//   many short rows: a block per row, no block of a few live threads at a row's end.
+//     5200 x 654, 3 layers 266: 299 / 278 / 261;  754 x 191, 12 layers 107: 115 / 110 / 107;
+//     272 x 573, 11 layers 110: 110 / 114 / 115.  Rows of one run are a block anyway:
+//     6761 x 121, 7 layers 210: 234 / 215 / 222
+//   a half-space alone: a solve is so short that a block wants many (70 x 4636 71: 76 / 76 / 71)
+//   few blocks: more registers, a shorter chain (165 x 766, 10 layers 89: 91 / 95 / 114);
+//     many: the fifth block (363 x 2367, 9 layers 189: 193 / 187 / 282)
+int direct_variant(int nl, long long rows, int nk) {
+    constexpr int kManyRows = 3 * 148, kManyRuns = 15 * 148, kManyLong = 240;
+    const long long runs = rows * ((nk + 127) / 128), longs = rows * ((nk + 128 * kRowSweeps - 1) / (128 * kRowSweeps));
+    if ((nk > 128 && nk <= 128 * kRowSweeps && rows >= kManyRows) || (nl == 1 && longs >= kManyLong)) return kPropFixed + 2;
+    return kPropFixed + (runs <= kManyRuns ? 0 : 1);
+}
+
 bool prop_variant_shape(int variant, int* threads, int* blocks_per_sm, int* ilp, int* sweeps, int* persistent) {
+    if (variant >= kPropFixed && variant < kPropFixed + kDirectCount) {
+        const DirectVariant& v = kDirectVariants[variant - kPropFixed];
+        *threads = v.threads;
+        *blocks_per_sm = v.minb;
+        *ilp = 1;
+        *sweeps = v.sweeps;
+        *persistent = 0;
+        return true;
+    }
     if (variant < 0 || variant >= kPropVariants) return false;
     const PropVariant& v = kDunkinVariants[variant];
     *threads = v.threads;
@@ -652,12 +695,11 @@ void launch_prop(cudaStream_t s, const LayerC* lc, const MediumP* media, const F
             k_prop<0, 128, 1, false, false><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
         return;
     }
-    if (variant == kPropDirect) {
-        const dim3 grid((max_nk + 127) / 128, nf);
-        if (slice)
-            k_prop<2, 128, 5, false, true><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
-        else
-            k_prop<2, 128, 5, false, false><<<grid, 128, 0, s>>>(lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
+    if (variant >= kPropFixed && variant < kPropFixed + kDirectCount) {
+        const DirectVariant& v = kDirectVariants[variant - kPropFixed];
+        const int per_block = v.threads * v.sweeps;
+        (slice ? v.fn_slice : v.fn)<<<dim3((max_nk + per_block - 1) / per_block, nf), v.threads, 0, s>>>(
+            lc, media, fd, wc2, C, tab, rem, status, so, PropQueue{});
         return;
     }
     if (variant < 0 || variant >= kPropVariants) variant = 0;
