@@ -27,7 +27,8 @@ struct gfk_weights {
     double dk = 0.0;   // wavenumber step
     std::vector<double> ranges;
     void* d = nullptr;
-    bool built = false;  // its build has been enqueued on the context's stream
+    bool built = false;         // its build has been enqueued on the context's stream
+    bool panels_built = false;  // the panel weights' too (kFused)
     bool same(Kind kind_, int n_, double dk_, const double* r, int nr) const {
         return kind == kind_ && n == n_ && dk == dk_ && (int)ranges.size() == nr &&
                std::equal(ranges.begin(), ranges.end(), r);

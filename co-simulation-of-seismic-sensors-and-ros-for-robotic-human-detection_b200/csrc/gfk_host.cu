@@ -203,10 +203,20 @@ struct TimedSeg {
 //   120 x 2428, 11 layers 123 / 159 us        670 x 1384, 6 layers 161 / 162 us
 //   109 x 8819, 3 layers 127 / 114 us         116 x 9695, 9 layers 222 / 205 us
 //   264 x 8419, 5 layers 259 / 209 us         324 x 15439, 9 layers 734 / 452 us
+// With the sum fused in, a panel's nodes are the whole of its work: long rows, whose fine
+// grids are all but never refused, and few layers have panels earlier:
+//   3 x 143115, 5 layers 199 / 66 us          10 x 78078, 6 layers 202 / 73 us
+//   56 x 13324, 2 layers 75 / 61 us           46 x 4573, 2 layers 50 / 58 us
+//   20 x 5065, 5 layers 57 / 90 us            57 x 8574, 10 layers 134 / 178 us
 // The plan's total decides, so its chunks agree, and a forced shape has panels.
-constexpr int64_t kDirectPoints = 950000;
-bool solves_every_point(int64_t rows, int nk) {
-    return (nk <= 128 * gfk::kRowSweeps || rows * nk <= kDirectPoints) && !getenv("GFK_PROP_VARIANT");
+constexpr int64_t kDirectPoints = 950000, kFusedDirectPoints = 150000;
+constexpr int kFusedDirectRow = 4096, kFusedDirectLongest = 10240;
+bool solves_every_point(int64_t rows, int nk, int nl, bool fused) {
+    if (getenv("GFK_PROP_VARIANT")) return false;
+    if (nk <= 128 * gfk::kRowSweeps) return true;
+    if (fused && (nk > std::min(kFusedDirectLongest, nl * kFusedDirectRow) || rows * nk > nl * kFusedDirectPoints))
+        return false;
+    return rows * nk <= kDirectPoints;
 }
 
 struct gfk_plan {
@@ -629,7 +639,14 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         p->fused = true;
         p->tc = false;
     }
-    p->direct = p->shared && !p->fused && s->formulation == GFK_DUNKIN && solves_every_point(p->nf, p->g_n);
+    p->direct = p->shared && s->formulation == GFK_DUNKIN && solves_every_point(p->nf, p->g_n, p->max_nl, p->fused);
+    // plans of one launch shape, nothing to tune
+    if (p->fused)
+        p->prop_variant = gfk::fused_variant(p->max_nl, p->nf, p->g_n, nr, p->direct);
+    else if (p->direct)
+        p->prop_variant = gfk::direct_variant(p->max_nl, p->nf, p->g_n);
+    else if (!p->shared)
+        p->prop_variant = s->formulation == GFK_DUNKIN ? gfk::kPropRows : 0;
     // row chunks bounded by the integrand budget and the grid limit; on a shared
     // grid every row keeps its dense slot (row x Nk), failed rows included
     const int64_t budget = kDefaultRemBudget / (int64_t)sizeof(cd);
@@ -700,7 +717,7 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         int max_cnf = 0;
         for (size_t c = 0; c + 1 < p->chunk_begin.size(); c++)
             max_cnf = std::max(max_cnf, p->chunk_begin[c + 1] - p->chunk_begin[c]);
-        const int nkb = (g_n + 1023) / 1024;
+        const int span = gfk::fused_span(p->prop_variant), nkb = (g_n + span - 1) / span;
         lay.add(&p->d_partial, (size_t)max_cnf * nkb * nr);
     } else {
         lay.add(&p->d_rem, (size_t)std::max<int64_t>(cap, 1));
@@ -755,13 +772,6 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
         if (p->chunk_begin[c + 1] > p->chunk_begin[c]) nchunks++;
     p->launches_per_exec = p->nf > 0 ? (p->shared ? 2 : 1) + 2 * nchunks : 0;
     if (p->nf > 0 && (p->ksplit > 1 || !p->shared)) p->launches_per_exec += nchunks;
-    // plans of one launch shape, nothing to tune
-    if (p->direct)
-        p->prop_variant = gfk::direct_variant(p->max_nl, p->nf, p->g_n);
-    else if (!p->shared && p->solve.formulation == GFK_DUNKIN)
-        p->prop_variant = gfk::kPropRows;
-    else if (p->fused || !p->shared)
-        p->prop_variant = 0;
     *out = p;
     return GFK_OK;
 }
@@ -929,11 +939,12 @@ int plan_enqueue(gfk_plan* p, bool timed) {
         else
             gfk::launch_j0_table(s, p->d_ranges, p->nr, p->g_n, p->g_kmax / p->g_n, p->d_W);
         ctx->launches++;
-        if (p->fused) {
-            gfk::launch_panel_weights(s, p->d_W, ctx->panels, p->g_n, p->nr, p->d_W + (size_t)p->g_n * p->nr);
-            ctx->launches++;
-        }
         p->wts->built = true;
+    }
+    if (p->fused && !p->direct && !p->wts->panels_built) {
+        gfk::launch_panel_weights(s, p->d_W, ctx->panels, p->g_n, p->nr, p->d_W + (size_t)p->g_n * p->nr);
+        ctx->launches++;
+        p->wts->panels_built = true;
     }
     if (timed && (st = end_seg(p, seg))) return st;
     ctx->launches += p->shared ? 2 : 1;
@@ -948,7 +959,7 @@ int plan_enqueue(gfk_plan* p, bool timed) {
             if (timed && (st = begin_seg(p, 0, &seg))) return st;
             gfk::launch_prop_fused(s, p->d_lc, p->d_media, p->d_fd + fb, p->d_wc2 + fb, cnf, p->g_n, p->d_C + fb,
                                    ctx->panels, p->d_W, p->d_W + (size_t)p->g_n * p->nr, p->d_ranges, p->nr,
-                                   p->d_partial, p->d_status + fb,
+                                   p->prop_variant, p->d_partial, p->d_status + fb,
                                    p->d_G + (size_t)fb * p->nr);
             if (timed && (st = end_seg(p, seg))) return st;
             ctx->launches += 2;

@@ -616,6 +616,18 @@ const DirectVariant kDirectVariants[] = {
 };
 constexpr int kDirectCount = sizeof(kDirectVariants) / sizeof(kDirectVariants[0]);
 #undef GFK_DIRECT
+static_assert(kPropFixed + kDirectCount == kPropFused, "fixed variants follow one another");
+
+// The launches with the sum fused in (k_prop_fused), variants kPropFused + index:
+// `sweeps` runs of 128 wavenumbers a block, or panels of 128.
+struct FusedVariant {
+    int minb, sweeps;
+    bool panel;
+};
+const FusedVariant kFusedVariants[] = {
+    {4, 1, false}, {4, 2, false}, {4, kRowSweeps, false}, {6, 8, true}, {4, 8, true},  // up to 2 ranges, up to 8
+};
+constexpr int kFusedCount = sizeof(kFusedVariants) / sizeof(kFusedVariants[0]);
 #undef GFK_PROP_SHAPE
 #undef GFK_PROP_QUEUE
 
@@ -666,6 +678,15 @@ bool prop_variant_shape(int variant, int* threads, int* blocks_per_sm, int* ilp,
     if (variant >= kPropFixed && variant < kPropFixed + kDirectCount) {
         const DirectVariant& v = kDirectVariants[variant - kPropFixed];
         *threads = v.threads;
+        *blocks_per_sm = v.minb;
+        *ilp = 1;
+        *sweeps = v.sweeps;
+        *persistent = 0;
+        return true;
+    }
+    if (variant >= kPropFused && variant < kPropFused + kFusedCount) {
+        const FusedVariant& v = kFusedVariants[variant - kPropFused];
+        *threads = 128;
         *blocks_per_sm = v.minb;
         *ilp = 1;
         *sweeps = v.sweeps;
@@ -740,11 +761,13 @@ void launch_prop_rows(cudaStream_t s, const LayerC* lc, const MediumP* media, co
 // tree, then warps), and one partial per (row, k block, range) is written. A
 // panel taken from its nodes is never interpolated: the weights of its 128
 // wavenumbers are carried over to the nodes once per grid (k_panel_weights).
+// Short rows and small plans (fused_variant) solve every wavenumber, 1, 2 or
+// kRowSweeps runs of 128 a block, and need no node weights.
 // The integrand never reaches HBM; k_fused_finish adds the partials in block
 // order (deterministic) and the closed k = 0 panel (fk.go:529-532).
 
 constexpr int kFuseThreads = 128;
-constexpr int kFuseSpan = 8 * kFuseThreads;  // wavenumbers of its row a block covers
+constexpr int kFuseSpan = 8 * kFuseThreads;  // wavenumbers of its row a block of panels covers
 
 // Wp[panel][48][nr]: sum over the panel's wavenumbers of the interpolation
 // matrix times W, for the 16-node and then the 32-node fit.
@@ -770,15 +793,17 @@ void launch_panel_weights(cudaStream_t s, const double* W, const double* tab, in
     k_panel_weights<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(W, tab, nk, nr, Wp);
 }
 
-template <int NR>
-__global__ __launch_bounds__(kFuseThreads, NR <= 2 ? 6 : 4) void k_prop_fused(const LayerC* __restrict__ lc,
+// PANEL: `sweeps` is not read; else the runs of 128 wavenumbers a block covers.
+template <int NR, bool PANEL>
+__global__ __launch_bounds__(kFuseThreads, PANEL && NR <= 2 ? 6 : 4) void k_prop_fused(const LayerC* __restrict__ lc,
                                                                 const MediumP* __restrict__ media,
                                                                 const FreqDesc* __restrict__ fd,
                                                                 const cd* __restrict__ wc2, const cd* __restrict__ C,
                                                                 const double* __restrict__ tab,
                                                                 const double* __restrict__ W,
                                                                 const double* __restrict__ Wp, int nr, int nkb,
-                                                                cd* __restrict__ partial, int* __restrict__ status) {
+                                                                int sweeps, cd* __restrict__ partial,
+                                                                int* __restrict__ status) {
     __shared__ PropSmem<kFuseThreads, false> sm;
     __shared__ double s_red[2 * NR][kFuseThreads / 32];
     const int f = gridDim.y - 1 - blockIdx.y;  // the costlier rows first
@@ -791,10 +816,28 @@ __global__ __launch_bounds__(kFuseThreads, NR <= 2 ? 6 : 4) void k_prop_fused(co
     double acc[2 * NR];
 #pragma unroll
     for (int q = 0; q < 2 * NR; q++) acc[q] = 0.0;
-    double mre = 0.0, mim = 0.0;
     int bad = 0;
-    panel_item<kFuseThreads, false, NR, true>(tab, sm, nl, med.mu_ref, wc2[f], C[f], fdesc.dk, n, blockIdx.x * kFuseSpan, n,
-                                       nullptr, W, Wp, nr, acc, mre, mim, bad);
+    if constexpr (PANEL) {
+        double mre = 0.0, mim = 0.0;
+        panel_item<kFuseThreads, false, NR, true>(tab, sm, nl, med.mu_ref, wc2[f], C[f], fdesc.dk, n,
+                                                  blockIdx.x * kFuseSpan, n, nullptr, W, Wp, nr, acc, mre, mim, bad);
+    } else {
+        const cd w2 = wc2[f], c = C[f];
+#pragma unroll 1
+        for (int sweep = 0; sweep < sweeps; sweep++) {
+            const int i = (blockIdx.x * sweeps + sweep) * kFuseThreads + threadIdx.x + 1;
+            if (i > n) break;
+            const double k = (double)i * fdesc.dk;
+            cd r = k * dunkin_u(sm.lc, nl, w2, k, med.mu_ref) - c;
+            if (!finite_cd(r)) { bad |= kStNonfinite; r = mk(0.0); }
+#pragma unroll
+            for (int q = 0; q < NR; q++) {
+                const double w = q < nr ? W[(size_t)(i - 1) * nr + q] : 0.0;
+                acc[2 * q] = fma(r.re, w, acc[2 * q]);
+                acc[2 * q + 1] = fma(r.im, w, acc[2 * q + 1]);
+            }
+        }
+    }
     if (bad) atomicOr(status + f, bad);
     // warp tree, then the block's warps in order: a fixed summation order
 #pragma unroll
@@ -827,26 +870,48 @@ __global__ void k_fused_finish(const cd* __restrict__ partial, const cd* __restr
     const cd c = C[f];
     const double d = fd[f].dk;
     cd acc = c / ranges[j] - (0.5 * d) * c;
+#pragma unroll 8
     for (int b = 0; b < nkb; b++) acc += partial[((size_t)f * nkb + b) * nr + j];
     G[(size_t)f * nr + j] = acc;
 }
 
 int fused_max_ranges() { return 8; }
 
+// Many short rows take a block each, rows of two runs earlier: as blocks of their own
+// a full and a nearly empty run alternate over the SMs. A solve of one or two finite layers is short
+// beside a block's table load and reduction: two runs a block there. Execute of a plan
+// with 1 / 2 / 4 / 8 runs a block (us):
+//   552 rows x 207, 8 layers 66 / 57 / 57 / 57    245 x 252, 9 layers 64 / 55 / 55 / 55
+//   141 x 359, 10 layers 60 / 70 / 66 / 66        283 x 760, 6 layers 68 / 70 / 82 / 67
+//   129 x 3608, 8 layers 115 / 118 / 128 / 201    25 x 5823, 4 layers 55 / 53 / 63 / 70
+//   21 x 4616, 2 layers 46 / 44 / 44 / 52         26 x 3437, half-space 43 / 39 / 39 / 42
+int fused_variant(int nl, long long rows, int nk, int nr, bool direct) {
+    constexpr int kManyRows = 400, kManyPairs = 148;
+    if (!direct) return kPropFused + (nr <= 2 ? 3 : 4);
+    const bool is_short = nk <= 128 * kRowSweeps;
+    return kPropFused + (is_short && rows >= (nk <= 256 ? kManyPairs : kManyRows) ? 2 : !is_short && nl <= 3 ? 1 : 0);
+}
+
+int fused_span(int variant) { return kFuseThreads * kFusedVariants[variant - kPropFused].sweeps; }
+
+namespace {
+template <int NR>
+void launch_fused(cudaStream_t s, dim3 grid, bool panel, const LayerC* lc, const MediumP* media, const FreqDesc* fd,
+                  const cd* wc2, const cd* C, const double* tab, const double* W, const double* Wp, int nr, int sweeps,
+                  cd* partial, int* status) {
+    (panel ? k_prop_fused<NR, true> : k_prop_fused<NR, false>)<<<grid, kFuseThreads, 0, s>>>(
+        lc, media, fd, wc2, C, tab, W, Wp, nr, (int)grid.x, sweeps, partial, status);
+}
+}  // namespace
+
 void launch_prop_fused(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, const cd* wc2,
                        int nf, int nk, const cd* C, const double* tab, const double* W, const double* Wp,
-                       const double* ranges, int nr, cd* partial, int* status, cd* G) {
+                       const double* ranges, int nr, int variant, cd* partial, int* status, cd* G) {
     if (nf <= 0 || nk <= 0 || nr <= 0 || nr > 8) return;
-    const int nkb = (nk + kFuseSpan - 1) / kFuseSpan;
-    dim3 grid(nkb, nf);
-    if (nr <= 1)
-        k_prop_fused<1><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, tab, W, Wp, nr, nkb, partial, status);
-    else if (nr <= 2)
-        k_prop_fused<2><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, tab, W, Wp, nr, nkb, partial, status);
-    else if (nr <= 4)
-        k_prop_fused<4><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, tab, W, Wp, nr, nkb, partial, status);
-    else
-        k_prop_fused<8><<<grid, kFuseThreads, 0, s>>>(lc, media, fd, wc2, C, tab, W, Wp, nr, nkb, partial, status);
+    const FusedVariant& v = kFusedVariants[variant - kPropFused];
+    const int span = fused_span(variant), nkb = (nk + span - 1) / span;
+    const auto fn = nr <= 1 ? launch_fused<1> : nr <= 2 ? launch_fused<2> : nr <= 4 ? launch_fused<4> : launch_fused<8>;
+    fn(s, dim3(nkb, nf), v.panel, lc, media, fd, wc2, C, tab, W, Wp, nr, v.sweeps, partial, status);
     const int64_t nt = (int64_t)nf * nr;
     k_fused_finish<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(partial, C, ranges, fd, nf, nr, nkb, G);
 }

@@ -56,6 +56,7 @@ void launch_prop(cudaStream_t s, const LayerC* lc, const MediumP* media, const F
 // plan of `rows` rows of nk wavenumbers and nl stack entries. Rows of up to
 // kRowSweeps x 128 wavenumbers are short.
 constexpr int kPropFixed = 64;
+constexpr int kPropFused = 67;  // to 71: the launches of launch_prop_fused
 constexpr int kPropRows = 1;  // the shape of launch_prop_rows' blocks of panels
 constexpr int kRowSweeps = 9;
 int direct_variant(int nl, long long rows, int nk);
@@ -87,14 +88,17 @@ int quad_tc_selftest_timeout(cudaStream_t s, long long wait_cycles, int* timed_o
 int quad_tc_splits(int M, int N, int Kp);  // split count filling the SMs for one chunk shape
 
 // Shared grid, nr <= fused_max_ranges(): propagator and wavenumber sum in one
-// pass (the integrand stays on chip); partial holds nf x ceil(nk/1024) x nr.
-// Wp: the weights carried over to the panels' nodes (launch_panel_weights).
+// pass (the integrand stays on chip); partial holds nf x ceil(nk / span) x nr.
+// Wp: the weights carried over to the panels' nodes (launch_panel_weights); a
+// `direct` variant, which solves every wavenumber, reads neither tab nor Wp.
 int fused_max_ranges();
+int fused_variant(int nl, long long rows, int nk, int nr, bool direct);
+int fused_span(int variant);  // wavenumbers of its row a block covers
 size_t panel_weight_count(int nk, int nr);
 void launch_panel_weights(cudaStream_t s, const double* W, const double* tab, int nk, int nr, double* Wp);
 void launch_prop_fused(cudaStream_t s, const LayerC* lc, const MediumP* media, const FreqDesc* fd, const cd* wc2,
                        int nf, int nk, const cd* C, const double* tab, const double* W, const double* Wp,
-                       const double* ranges, int nr, cd* partial, int* status, cd* G);
+                       const double* ranges, int nr, int variant, cd* partial, int* status, cd* G);
 
 // W[(i-1) nr + j] = w_i J0(k_i r_j) dk, w = 1/2 at i = nk.
 void launch_j0_table(cudaStream_t s, const double* ranges, int nr, int nk, double dk, double* W);

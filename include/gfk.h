@@ -230,18 +230,19 @@ int32_t gfk_plan_launches_per_execute(const gfk_plan *p);
 /* The plan's first execute times each launch shape of the Dunkin propagator
  * (gfk_prop_shape) on a window of up to 1024 of its own frequencies and keeps
  * the fastest; the context remembers the choice
- * per (layer count, wavenumber count) for later plans and calls. A shared grid of more
- * than 8 ranges with at most 1152 wavenumbers, or at most 950000 (frequency, wavenumber)
- * points, solves every point in a shape fixed by its size (64 to 66); grids that
- * differ per frequency have shape 1. Neither times any, nor does a sum that
- * is fused into the propagator (1 to 8 ranges). The environment variable
- * GFK_PROP_VARIANT=<index> forces a shape below 64 on shared grids of more than
- * 8 ranges instead. Writes the chosen index and up
- * to `capacity` measured times (ms); returns the number of shapes timed. */
+ * per (layer count, wavenumber count) for later plans and calls. Plans whose shape
+ * follows from their size time none: a shared grid of more than 8 ranges with
+ * at most 1152 wavenumbers, or at most 950000 (frequency, wavenumber) points, solves every
+ * point (shapes 64 to 66); with 1 to 8 ranges the sum is fused into the propagator
+ * (67 to 69 solve every point, 70 and 71 panels' nodes); grids that differ per
+ * frequency have shape 1. The environment variable GFK_PROP_VARIANT=<index> forces a shape
+ * below 64 on shared grids of more than 8 ranges, and panels with fewer. Writes the
+ * chosen index and up to `capacity` measured times (ms); returns the number of shapes
+ * timed. */
 int gfk_plan_tuning(const gfk_plan *p, int32_t *variant, float *ms_per_variant, int32_t capacity);
 /* Launch shape `variant` of the Dunkin propagator: threads per block, the
- * blocks per SM it is compiled for, wavenumbers per thread at a time, panels (from
- * 64 on, where every wavenumber is solved: runs) of 128 wavenumbers per work item, and
+ * blocks per SM it is compiled for, wavenumbers per thread at a time, panels (64 to
+ * 69, where every wavenumber is solved: runs) of 128 wavenumbers per work item, and
  * whether it is persistent (one
  * block per resident slot taking (row, item) pairs from a device queue, the last
  * rows first; otherwise one item per block). GFK_EARG for an unknown index. */
