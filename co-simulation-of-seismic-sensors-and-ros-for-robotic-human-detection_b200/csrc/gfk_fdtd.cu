@@ -15,8 +15,8 @@
 // that loads a tile and a halo of S cells can take S steps in shared memory
 // before it writes its tile back (k_tiles): one launch and one pass over memory
 // per S steps. The fields are double-buffered, because neighbouring tiles read
-// what this one writes. Where the second copy does not fit the device, each
-// phase is one kernel over the grid in place (k_velocities, which also writes
+// what this one writes. Where the second copy does not fit the device (or
+// GFK_FDTD_COPIES=1 asks for one), each phase is one kernel over the grid in place (k_velocities, which also writes
 // the prescribed surface traction, and k_stresses, which also records the
 // receivers: their velocities are final by then). The arithmetic of every cell is the
 // reference's, in the same order, except that divisions by the spacing, the
@@ -25,6 +25,7 @@
 // reduction checks for divergence, as Run does.
 #include <cmath>
 #include <complex>
+#include <cstdlib>
 #include <string>
 #include <utility>
 #include <vector>
@@ -44,7 +45,7 @@ struct Args {
     bool lossy;
     double mem_decay, mem_drive;
     // materials per row; the time step over the densities, precomputed
-    const double *rho, *lamU, *muU, *rhoZ, *muZ;
+    const double *lamU, *muU, *muZ;
     const double *dt_rho, *dt_rhoZ;
     // reciprocal spacings and radii: 1 / dr, 1 / dz, 1 / ((i + 1/2) dr), 1 / (i dr)
     double idr, idz;
@@ -694,10 +695,8 @@ int gfk_fdtd_run(gfk_ctx* ctx, const gfk_fdtd_model* md, const double* force, in
     up(dtrz, &a.dt_rhoZ);
     up(irh, &a.ir_half);
     up(iri, &a.ir_int);
-    up(rho, &a.rho);
     up(lamU, &a.lamU);
     up(muU, &a.muU);
-    up(rhoZ, &a.rhoZ);
     up(muZ, &a.muZ);
     up(pRi.a, &a.aRi);
     up(pRi.b, &a.bRi);
@@ -718,19 +717,29 @@ int gfk_fdtd_run(gfk_ctx* ctx, const gfk_fdtd_model* md, const double* force, in
     auto has = [&](int f) { return a.lossy || f < gfk::fdtd::kRrr || f > gfk::fdtd::kRrz; };
     const int nfield = gfk::fdtd::kFields - (a.lossy ? 0 : 4);
     // two copies of the fields, where they take at most half of what is free
-    // (asked only for large grids: the query takes up to a millisecond)
+    // (asked only for large grids: the query takes up to a millisecond) and can be
+    // had; else one. GFK_FDTD_COPIES=<1 or 2> replaces the question.
     gfk::fdtd::Tiles tl{};
     size_t mem_free = 0, mem_all = 0;
-    const bool fits = 2 * n * 8 * nfield <= (size_t(1) << 30) ||
-                      (cudaMemGetInfo(&mem_free, &mem_all) == cudaSuccess && 2 * n * 8 * nfield <= mem_free / 2);
-    const bool tiled = fits &&
-                       cudaFuncSetAttribute(a.lossy ? gfk::fdtd::k_tiles<true> : gfk::fdtd::k_tiles<false>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            gfk::fdtd::kTileSmem) == cudaSuccess;
+    const char* asked = getenv("GFK_FDTD_COPIES");
+    const bool fits = asked ? atoi(asked) > 1
+                            : 2 * n * 8 * nfield <= (size_t(1) << 30) ||
+                                  (cudaMemGetInfo(&mem_free, &mem_all) == cudaSuccess && 2 * n * 8 * nfield <= mem_free / 2);
+    bool tiled = fits && cudaFuncSetAttribute(a.lossy ? gfk::fdtd::k_tiles<true> : gfk::fdtd::k_tiles<false>,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              gfk::fdtd::kTileSmem) == cudaSuccess;
     std::vector<double> fpad(force, force + std::max(0, std::min(nforce, steps + 1)));
     fpad.resize((size_t)steps + 1, 0.0);
-    const size_t copy = (n * 8 + 255) / 256 * 256, all = (tiled ? 2 : 1) * nfield * copy;
+    const size_t copy = (n * 8 + 255) / 256 * 256;
+    size_t all = (tiled ? 2 : 1) * nfield * copy;
     unsigned char* slab = static_cast<unsigned char*>(dev(all));
+    if (!slab && tiled) {
+        cudaGetLastError();
+        owned.clear();
+        tiled = false;
+        all = nfield * copy;
+        slab = static_cast<unsigned char*>(dev(all));
+    }
     for (int f = 0, at = 0; slab && f < gfk::fdtd::kFields; f++)
         if (has(f)) {
             *fields[f] = reinterpret_cast<double*>(slab + at * copy);

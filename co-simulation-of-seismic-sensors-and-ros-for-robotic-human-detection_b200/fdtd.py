@@ -3,8 +3,8 @@
 Same names and behaviour as the Go package: Model (model.go:30-100), Ricker
 and RickerSpectrum (run.go:14-44), Shot / Trace / Result / Run
 (run.go:46-127), SpacingFor (model.go:102-120). Run executes every time
-step on the device (gfk_fdtd_run: one velocity and one stress kernel per
-step over the whole grid) and returns the surface traces.
+step on the device (gfk_fdtd_run: several steps per launch in tiles of the
+grid) and returns the surface traces.
 """
 import ctypes
 import math
