@@ -46,9 +46,12 @@ struct gfk_ctx {
     std::vector<gfk_dataset*> datasets;  // live surrogate data sets and networks,
     std::vector<gfk_net*> nets;          // destroyed by gfk_close as well
     std::vector<gfk_bank_dev*> banks;    // device-resident banks (gfk_consume.cu)
-    // propagator launch shape chosen by tuning, per (layer count, wavenumber count)
+    // propagator launch shape chosen by tuning, per (layer count, wavenumber count, with
+    // the tensor-core sum's slicing or not, few items or many)
     struct Tuned {
-        int nl, nk, variant;
+        int nl, nk;
+        bool tc, few;
+        int variant;
     };
     std::vector<Tuned> tuned;
     // tensor-core sum tile shape chosen by tuning, per padded (rows, ranges, wavenumbers)

@@ -788,11 +788,18 @@ gfk::RowItems row_items(const gfk_plan* p, int fb, int n) {
     return gfk::RowItems{p->d_item_row + i0, p->d_row_begin + fb, fb, i0, p->row_begin[fb + n] - i0, p->kc};
 }
 
+// Items of 8 panels in a window up to which another shape leads than above. With few,
+// the SMs are not full and the shapes of shorter items win, all nodes at once above all:
+// with 11 layers and 3001 wavenumbers 317 rows took 140 us in the fastest shape of that
+// kind and 188 in the fastest of the others, 5072 rows 1724 and 1475 us; 634 rows (1902 items)
+// are within 10% either way. Over 2 to 11 layers and 1200 to 40000 wavenumbers the shapes
+// swap places between 1900 and 3700 items.
+constexpr int kTuneFewItems = 2500;
+
 // Times every Dunkin launch shape on a window of up to 1024 rows of the first
-// chunk (its middle) and keeps the fastest. Small windows rank the shapes
-// by their launch tails: 64 rows could not tell shapes 4% apart at full size,
-// and 256 rows ranked the shapes with several wavenumber runs per block last
-// although they are the fastest on the graded soil's 2048 rows. The window's
+// chunk (its middle) and keeps the fastest; the context remembers it for later plans of as
+// many layers and wavenumbers, the same kind of sum and few or many items alike. Small
+// windows rank the shapes by their launch tails. The window's
 // integrand rows are recomputed by the real launch afterwards.
 int tune_prop(gfk_plan* p) {
     gfk_ctx* ctx = p->ctx;
@@ -804,14 +811,15 @@ int tune_prop(gfk_plan* p) {
         return GFK_OK;
     }
     if (p->solve.formulation != GFK_DUNKIN || p->nf == 0) return GFK_OK;
-    for (const auto& t : ctx->tuned)
-        if (t.nl == p->max_nl && t.nk == p->max_nk) {
-            p->prop_variant = t.variant;
-            return GFK_OK;
-        }
     const int c0 = p->chunk_begin[0], c1 = p->chunk_begin[1];
     const int win = std::min(1024, c1 - c0);
     if (win <= 0) return GFK_OK;
+    const bool few = (int64_t)win * ((p->max_nk + 8 * gfk::kPanel - 1) / (8 * gfk::kPanel)) <= kTuneFewItems;
+    for (const auto& t : ctx->tuned)
+        if (t.nl == p->max_nl && t.nk == p->max_nk && t.tc == p->tc && t.few == few) {
+            p->prop_variant = t.variant;
+            return GFK_OK;
+        }
     const int fb = c0 + (c1 - c0 - win) / 2;
     int cmax = 0;
     for (int f = fb; f < fb + win; f++) cmax = std::max(cmax, p->fd[f].kfar > 0 ? p->fd[f].nk : 0);
@@ -848,7 +856,7 @@ int tune_prop(gfk_plan* p) {
     for (int v = 1; v < nv; v++)
         if (p->tune_ms[v] < p->tune_ms[best]) best = v;
     p->prop_variant = best;
-    ctx->tuned.push_back({p->max_nl, p->max_nk, best});
+    ctx->tuned.push_back({p->max_nl, p->max_nk, p->tc, few, best});
     return GFK_OK;
 }
 

@@ -230,7 +230,8 @@ int32_t gfk_plan_launches_per_execute(const gfk_plan *p);
 /* The plan's first execute times each launch shape of the Dunkin propagator
  * (gfk_prop_shape) on a window of up to 1024 of its own frequencies and keeps
  * the fastest; the context remembers the choice
- * per (layer count, wavenumber count) for later plans and calls. Plans whose shape
+ * per layer count, wavenumber count, kind of sum and few or many items (2500 of 1024
+ * wavenumbers in the window) for later plans and calls. Plans whose shape
  * follows from their size time none: a shared grid of more than 8 ranges with
  * at most 1152 wavenumbers, or at most 950000 (frequency, wavenumber) points, solves every
  * point (shapes 64 to 66); with 1 to 8 ranges the sum is fused into the propagator
