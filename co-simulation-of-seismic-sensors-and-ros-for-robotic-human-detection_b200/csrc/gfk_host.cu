@@ -644,7 +644,7 @@ int plan_build(gfk_ctx* ctx, const SoilIn* soils, int nsoil, const gfk_solve* s,
     if (p->fused)
         p->prop_variant = gfk::fused_variant(p->max_nl, p->nf, p->g_n, nr, p->direct);
     else if (p->direct)
-        p->prop_variant = gfk::direct_variant(p->max_nl, p->nf, p->g_n);
+        p->prop_variant = gfk::direct_variant(p->max_nl, p->nf, p->g_n, p->tc);
     else if (!p->shared)
         p->prop_variant = s->formulation == GFK_DUNKIN ? gfk::kPropRows : 0;
     // row chunks bounded by the integrand budget and the grid limit; on a shared

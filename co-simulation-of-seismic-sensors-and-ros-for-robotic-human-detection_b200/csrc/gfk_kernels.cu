@@ -157,7 +157,7 @@ void launch_static(cudaStream_t s, const LayerC* lc, const MediumP* media, const
 // Launch shapes are template parameters; the plan times them once and keeps
 // the fastest. The direct formulation (FORM 0) solves every wavenumber: its parity with
 // the reference includes the digits its eigenbasis loses. So does FORM 2, the Dunkin
-// solve of short rows and small banks (direct_variant), SWEEPS runs of 128
+// solve of short rows and small banks (direct_variant), SWEEPS runs of THREADS
 // wavenumbers a block, a wavenumber per thread in each.
 
 constexpr int kNodeStride = kPanelN + 4;  // of the node values in shared memory: conflict-free B fragments
@@ -608,11 +608,12 @@ struct DirectVariant {
     PropFn fn, fn_slice;
     int threads, minb, sweeps;
 };
-#define GFK_DIRECT(B, S) {k_prop<2, 128, B, false, false, S>, k_prop<2, 128, B, false, true, S>, 128, B, S}
+#define GFK_DIRECT(T, B, S) {k_prop<2, T, B, false, false, S>, k_prop<2, T, B, false, true, S>, T, B, S}
 const DirectVariant kDirectVariants[] = {
-    GFK_DIRECT(4, 1),           // <= 128 registers
-    GFK_DIRECT(5, 1),           // <= 96 registers
-    GFK_DIRECT(5, kRowSweeps),  // a short row per block
+    GFK_DIRECT(128, 4, 1),           // <= 128 registers
+    GFK_DIRECT(128, 5, 1),           // <= 96 registers
+    GFK_DIRECT(128, 5, kRowSweeps),  // a short row per block
+    GFK_DIRECT(256, 2, 1),           // <= 128 registers
 };
 constexpr int kDirectCount = sizeof(kDirectVariants) / sizeof(kDirectVariants[0]);
 #undef GFK_DIRECT
@@ -657,21 +658,42 @@ bool prop_variant_persistent(int variant) {
     return variant >= 0 && variant < kPropVariants && kDunkinVariants[variant].persistent;
 }
 
-// Which of kDirectVariants a plan of `rows` rows of nk wavenumbers takes. Plan execute on
-// either side of each line (us; first the fastest of the 13 shapes that used to be timed
-// for each plan, then these three in turn):
-//   many short rows: a block per row, no block of a few live threads at a row's end.
-//     5200 x 654, 3 layers 266: 299 / 278 / 261;  754 x 191, 12 layers 107: 115 / 110 / 107;
-//     272 x 573, 11 layers 110: 110 / 114 / 115.  Rows of one run are a block anyway:
-//     6761 x 121, 7 layers 210: 234 / 215 / 222
-//   a half-space alone: a solve is so short that a block wants many (70 x 4636 71: 76 / 76 / 71)
-//   few blocks: more registers, a shorter chain (165 x 766, 10 layers 89: 91 / 95 / 114);
-//     many: the fifth block (363 x 2367, 9 layers 189: 193 / 187 / 282)
-int direct_variant(int nl, long long rows, int nk) {
-    constexpr int kManyRows = 3 * 148, kManyRuns = 15 * 148, kManyLong = 240;
-    const long long runs = rows * ((nk + 127) / 128), longs = rows * ((nk + 128 * kRowSweeps - 1) / (128 * kRowSweeps));
-    if ((nk > 128 && nk <= 128 * kRowSweeps && rows >= kManyRows) || (nl == 1 && longs >= kManyLong)) return kPropFixed + 2;
-    return kPropFixed + (runs <= kManyRuns ? 0 : 1);
+// Which of kDirectVariants a plan of `rows` rows of nk wavenumbers takes. Execute of a
+// plan as a graph, on either side of each line (us; first the fastest of the 13 shapes that
+// used to be timed for each plan, then these four in turn; 2 us are one tick of the timer):
+//   rows of two runs: 256 threads hold one while every block is resident (two on each of 148
+//     SMs), then a block per row. 157 x 208, 12 layers 70: 76 / 76 / 72 / 70;
+//     538 x 166, 9 layers 69: 76 / 78 / 70 / 78;  2412 x 186, 9 layers 138: 150 / 142 / 132 / 186
+//   many short rows: a block per row, no block of a few live threads at a row's end. The
+//     longer the rows the later, as few rows are few blocks; with the split sum, whose
+//     last block of a row cuts its digits, earlier. 423 x 488, 7 layers, split 69: 74 / 72 / 68 / 76;
+//     403 x 469, 5 layers 80: 82 / 81 / 82 / 84;  564 x 1118, 2 layers, split 68: 74 / 70 / 64 / 79;
+//     467 x 1046, 9 layers, split 123: 125 / 121 / 132 / 131;  755 x 1050, 4 layers 99: 103 / 99 / 109 / 109;
+//     2590 x 964, 5 layers 360: 378 / 363 / 356 / 389
+//   rows of four runs, plain sum: two blocks of 256 threads from the second wave on
+//     (175 x 422, 12 layers 84: 89 / 96 / 96 / 84)
+//   a half-space alone: a solve is so short that a block wants many (112 x 4150, split 54:
+//     65 / 65 / 56 / 65)
+//   rows of one run: five blocks per SM where four leave a second wave, and for many
+//     (740 x 100, 8 layers, split 73: 70 / 62 / 63 / 84;  800 x 100 74: 72 / 74 / 74 / 89;
+//     1332 x 100 86: 84 / 76 / 78 / 113)
+//   long rows, few of them, split: 256 threads cut a row's digits (33 x 2608, 12 layers 74:
+//     78 / 84 / 176 / 72;  21 x 10767, 3 layers 69: 73 / 74 / 94 / 68)
+//   else few blocks: more registers, a shorter chain (91 x 1477, 11 layers, split 77: 76 / 80 /
+//     135 / 77); many: the fifth block (113 x 1553, 10 layers, split 84: 84 / 80 / 141 / 88)
+// Over 400 random plans the geometric mean is 1.004 of the fastest shape's speed, 0.998 with
+// 128 threads only and one line for all short rows; below 0.96 are 15 instead of 36.
+int direct_variant(int nl, long long rows, int nk, bool split) {
+    constexpr int kRun = 128, kShort = kRun * kRowSweeps, kManyLong = 240;
+    const long long runs = rows * ((nk + kRun - 1) / kRun), longs = rows * ((nk + kShort - 1) / kShort);
+    enum { kFew = kPropFixed, kMany, kRow, kPair };
+    if (nk <= kRun) return runs <= 4 * 148 || (runs > 5 * 148 && runs <= 8 * 148) ? kFew : kMany;
+    if (nk <= 2 * kRun) return rows <= 2 * 148 ? kPair : kRow;
+    if (nk <= kShort && rows >= (nk <= 4 * kRun ? 400 : split ? 540 : 1000)) return kRow;
+    if (nl == 1 && longs >= kManyLong) return kRow;
+    if (!split && nk > 3 * kRun && nk <= 4 * kRun && runs > 4 * 148 && runs <= 8 * 148) return kPair;
+    if (split && nk > 16 * kRun && runs > 3 * 148 && runs <= 13 * 148) return kPair;
+    return runs <= 8 * 148 ? kFew : kMany;
 }
 
 bool prop_variant_shape(int variant, int* threads, int* blocks_per_sm, int* ilp, int* sweeps, int* persistent) {

@@ -53,18 +53,18 @@ void launch_prop(cudaStream_t s, const LayerC* lc, const MediumP* media, const F
                  int max_nk, const cd* C, int formulation, const double* tab, cd* rem, int* status, int variant = 0,
                  const SliceOut* slice = nullptr, unsigned int* queue = nullptr);
 // Variants from kPropFixed on solve every wavenumber; direct_variant picks one for a
-// plan of `rows` rows of nk wavenumbers and nl stack entries. Rows of up to
+// plan of `rows` rows of nk wavenumbers and nl stack entries, with the split sum or not. Rows of up to
 // kRowSweeps x 128 wavenumbers are short.
 constexpr int kPropFixed = 64;
-constexpr int kPropFused = 67;  // to 71: the launches of launch_prop_fused
+constexpr int kPropFused = 68;  // to 72: the launches of launch_prop_fused
 constexpr int kPropRows = 1;  // the shape of launch_prop_rows' blocks of panels
 constexpr int kRowSweeps = 9;
-int direct_variant(int nl, long long rows, int nk);
+int direct_variant(int nl, long long rows, int nk, bool split);
 int prop_variant_count();
 bool prop_variant_persistent(int variant);
 // threads per block, blocks per SM it is compiled for, wavenumbers per thread
-// at a time, panels (or, solving every wavenumber, runs) of 128 wavenumbers per
-// item, persistent or one item per block
+// at a time, panels of 128 wavenumbers (or, solving every wavenumber, runs of a
+// wavenumber per thread) per item, persistent or one item per block
 bool prop_variant_shape(int variant, int* threads, int* blocks_per_sm, int* ilp, int* sweeps, int* persistent);
 
 // Tensor-core quadrature (gfk_quad_tc.cu): exact int8 slices of the integrand

@@ -234,16 +234,16 @@ int32_t gfk_plan_launches_per_execute(const gfk_plan *p);
  * wavenumbers in the window) for later plans and calls. Plans whose shape
  * follows from their size time none: a shared grid of more than 8 ranges with
  * at most 1152 wavenumbers, or at most 950000 (frequency, wavenumber) points, solves every
- * point (shapes 64 to 66); with 1 to 8 ranges the sum is fused into the propagator
- * (67 to 69 solve every point, 70 and 71 panels' nodes); grids that differ per
+ * point (shapes 64 to 67); with 1 to 8 ranges the sum is fused into the propagator
+ * (68 to 70 solve every point, 71 and 72 panels' nodes); grids that differ per
  * frequency have shape 1. The environment variable GFK_PROP_VARIANT=<index> forces a shape
  * below 64 on shared grids of more than 8 ranges, and panels with fewer. Writes the
  * chosen index and up to `capacity` measured times (ms); returns the number of shapes
  * timed. */
 int gfk_plan_tuning(const gfk_plan *p, int32_t *variant, float *ms_per_variant, int32_t capacity);
 /* Launch shape `variant` of the Dunkin propagator: threads per block, the
- * blocks per SM it is compiled for, wavenumbers per thread at a time, panels (64 to
- * 69, where every wavenumber is solved: runs) of 128 wavenumbers per work item, and
+ * blocks per SM it is compiled for, wavenumbers per thread at a time, panels of 128
+ * wavenumbers (64 to 70, where every wavenumber is solved: runs of a wavenumber per thread) per work item, and
  * whether it is persistent (one
  * block per resident slot taking (row, item) pairs from a device queue, the last
  * rows first; otherwise one item per block). GFK_EARG for an unknown index. */
