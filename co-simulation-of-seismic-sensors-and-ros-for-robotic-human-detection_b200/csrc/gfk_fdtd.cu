@@ -193,7 +193,7 @@ __global__ void k_stresses(Args s, double dTdt, int step) {
 // Cells of the window's rim lack a neighbour and are skipped, which is what the
 // shrinking accounts for. With every field in shared memory a step read and
 // wrote it 50 times a cell and its bandwidth bound the step. On a
-// 281 x 201 grid one launch per phase left 14.9 us a step, nearly all launch
+// 281 x 201 grid one launch per phase left 13.6 us a step, nearly all launch
 // and L2 latency on 382 cells an SM; on 6 million cells the two phases moved
 // 208 bytes a cell and step, here 220 per 4 steps.
 
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tiles(Args s, Tiles t) {
 // about 8 us for its window's loads and stores and 2.1 per step (fitted on one
 // wave of tiles, S = 2 to 8), times its waves of one tile per SM of 148. On
 // 281 x 201 cells S = 2, 3, 4, 5, 6 took 6.3, 4.6, 4.2, 4.2, 5.9 us a step, on 6.1
-// million cells 223, 208, 209, 228, 259; one launch per phase 13.8 and 322.
+// million cells 223, 208, 209, 228, 259; one launch per phase 13.6 and 321.
 int tile_steps(int nr, int nz) {
     int best = 1;
     double least = INFINITY;

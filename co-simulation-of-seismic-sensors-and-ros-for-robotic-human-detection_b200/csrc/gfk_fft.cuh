@@ -1,7 +1,8 @@
-// gfk_fft.cuh — FP64 complex radix-2 FFT of one power-of-two record in shared
-// memory, by the block that calls it.
+// gfk_fft.cuh — FP64 complex FFTs of one power-of-two record in shared
+// memory, by the block that calls it: fft_pow2 by radix-2 passes between two
+// buffers, fft_block by radix-8 passes through registers in one.
 //
-// The autosort (Stockham) formulation of Govindaraju et al., SC 2008: at the
+// fft_pow2 is the autosort (Stockham) formulation of Govindaraju et al., SC 2008: at the
 // stage with sub-transform length ns, butterfly j (< n/2) reads x[j] and
 // x[j + n/2] and writes y[2 ns (j / ns) + j % ns] and that + ns, with twiddle
 // e^{-2 pi i (j % ns) / (2 ns)} = tw[(j % ns) (n / (2 ns))], tw[m] =
