@@ -347,7 +347,10 @@ int gfk_fdtd_grid(const gfk_fdtd_model *m, double *dt, int32_t *nr, int32_t *nz)
  * ranges; meta (host, 5): dt, t0 (= dt/2, the velocities' time offset), the
  * largest particle speed seen, nr, nz. GFK_ENONFINITE with the reference's
  * message when the run diverges; GFK_EARG for a receiver outside the
- * interior or non-positive steps, spacing or domain. */
+ * interior or non-positive steps, spacing or domain. Two copies of the fields
+ * are kept where they take at most half of what is free (or 1 GiB) and can be had,
+ * else one, at a launch per phase of a step; the environment variable
+ * GFK_FDTD_COPIES=<1 or 2> replaces the first question. */
 int gfk_fdtd_run(gfk_ctx *ctx, const gfk_fdtd_model *m, const double *force, int32_t nforce,
                  const double *ranges_m, int32_t nrcv, int32_t steps, double *traces, double *snapped,
                  double *meta);
